@@ -145,42 +145,50 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
 
-// Returns false if the wait gave up (after limitNs of spinning) or another
-// block already failed.
+// One thread's arrival at the barrier and its wait.  Returns false if the
+// wait gave up (after limitNs of spinning) or another block already failed.
+__device__ __forceinline__ bool barrier_arrive_wait(unsigned* counter, unsigned target, int* err,
+                                                    unsigned long long limitNs = kBarrierNs) {
+    // the release orders the block's writes (made before the __syncthreads
+    // that precedes this call) ahead of the arrival; the wait polls relaxed
+    // (an acquire a poll costs more than the one that follows) and looks at
+    // the error word now and then only, since that is a second round trip to
+    // the L2; the closing acquire load orders the reads after it, and the
+    // __syncthreads that follows extends both to the whole block
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+    unsigned long long t0 = 0;
+    unsigned spins = 0;
+    while (ld_relaxed_u32(counter) < target) {
+        if (((++spins) & 63u) == 0) {
+            if (*(volatile int*)err != 0) return false;
+            unsigned long long t = globaltimer_ns();
+            if (t0 == 0) t0 = t;
+            else if (t - t0 > limitNs || spins > (1u << 30)) {
+                atomicCAS(err, 0, (int)CP_ERR_TIMEOUT);
+                return false;
+            }
+        }
+    }
+    (void)ld_acquire_u32(counter);
+    return true;
+}
+
 __device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned target, int* err,
                                              unsigned long long limitNs = kBarrierNs) {
     __shared__ int s_ok;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        // release pattern: the acq_rel fence orders the block's writes (made
-        // before the __syncthreads above) ahead of the relaxed arrival; the
-        // acquire loads below order the reads after it, and the closing
-        // __syncthreads extends both to the whole block
-        asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-        unsigned long long t0 = 0;
-        unsigned spins = 0;
-        while (ld_acquire_u32(counter) < target) {
-            if (((++spins) & 255u) == 0) {
-                unsigned long long t = globaltimer_ns();
-                if (t0 == 0) t0 = t;
-                else if (t - t0 > limitNs || spins > (1u << 30)) {
-                    atomicCAS(err, 0, (int)CP_ERR_TIMEOUT);
-                    ok = 0;
-                    break;
-                }
-            }
-            if (*(volatile int*)err != 0) { ok = 0; break; }
-        }
-        s_ok = ok;
-    }
+    if (threadIdx.x == 0) s_ok = barrier_arrive_wait(counter, target, err, limitNs) ? 1 : 0;
     __syncthreads();
     return s_ok != 0;
 }
@@ -205,6 +213,55 @@ __device__ __forceinline__ Team grid_team(unsigned* bar, int* err) {
 __device__ __forceinline__ bool team_sync(const Team& T, unsigned& target) {
     target += (unsigned)T.size;
     return grid_barrier(T.bar, target, T.err);
+}
+
+// Sum of NV values over the team, on the barrier that the sum needs anyway:
+// two block barriers in all (a block sum, a grid barrier and a sum of partials
+// one after the other take nine).  Warp 0 adds the block's warp sums, publishes
+// them, waits, and adds the team's partials; every thread gets the totals.
+// Fixed order, so the same inputs give the same bits on every run.  part: 4
+// doubles a CTA; the two halves alternate with the barrier count, so a slot is
+// rewritten only after every CTA has passed a later barrier.  sm: kReduceSm
+// doubles, written by team_reduce alone.
+constexpr int kReduceSm = 68;
+template <int NV>
+__device__ __forceinline__ bool team_reduce(const Team& T, unsigned& target, double (&v)[NV], double* part,
+                                            double* sm) {
+    static_assert(NV >= 1 && NV <= 2, "two values at most");
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    target += (unsigned)T.size;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        v[k] = warp_sum(v[k]);
+        if (lane == 0) sm[k * 32 + wid] = v[k];
+    }
+    __syncthreads();
+    if (wid == 0) {
+        double* slot = part + ((target / (unsigned)T.size) & 1u) * 2 * T.size;
+        double t[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            t[k] = warp_sum(lane < nw ? sm[k * 32 + lane] : 0.0);
+            if (lane == 0) __stcg(slot + NV * T.rank + k, t[k]);
+        }
+        int ok = 1;
+        if (lane == 0) ok = barrier_arrive_wait(T.bar, target, T.err) ? 1 : 0;
+        __syncwarp();
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            t[k] = 0.0;
+            if (ok)
+                for (int b = lane; b < T.size; b += 32) t[k] += __ldcg(slot + NV * b + k);
+            t[k] = warp_sum(t[k]);
+            if (lane == 0) sm[64 + k] = t[k];
+        }
+        if (lane == 0) sm[66] = (double)ok;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = sm[64 + k];
+    return sm[66] != 0.0;
 }
 
 __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* addr, double v) {
@@ -238,6 +295,50 @@ __device__ __forceinline__ Vec16<TV> zero16() {
     Vec16<TV> a;
 #pragma unroll
     for (int k = 0; k < Vec16<TV>::n; ++k) a.v[k] = (TV)0;
+    return a;
+}
+
+// V consecutive elements of one row (4, 8 or 16 bytes, aligned to their size)
+template <typename TV, int V>
+struct VecN {
+    TV v[V];
+};
+template <int V, typename TV>
+__device__ __forceinline__ VecN<TV, V> ldv(const TV* p) {
+    VecN<TV, V> o;
+    constexpr int B = V * (int)sizeof(TV);
+    static_assert(B == 4 || B == 8 || B == 16, "4, 8 or 16 bytes");
+    if constexpr (V == 1) {
+        o.v[0] = *p;
+    } else if constexpr (B == 8) {
+        const float2 f = *reinterpret_cast<const float2*>(p);
+        o.v[0] = f.x; o.v[1] = f.y;
+    } else {
+        const Vec16<TV> a = ld16(p);
+#pragma unroll
+        for (int k = 0; k < V; ++k) o.v[k] = a.v[k];
+    }
+    return o;
+}
+template <typename TV, int V>
+__device__ __forceinline__ void stv(TV* p, const VecN<TV, V>& a) {
+    constexpr int B = V * (int)sizeof(TV);
+    if constexpr (V == 1) {
+        *p = a.v[0];
+    } else if constexpr (B == 8) {
+        *reinterpret_cast<float2*>(p) = make_float2(a.v[0], a.v[1]);
+    } else {
+        Vec16<TV> o;
+#pragma unroll
+        for (int k = 0; k < V; ++k) o.v[k] = a.v[k];
+        st16(p, o);
+    }
+}
+template <typename TV, int V>
+__device__ __forceinline__ VecN<TV, V> zerov() {
+    VecN<TV, V> a;
+#pragma unroll
+    for (int k = 0; k < V; ++k) a.v[k] = (TV)0;
     return a;
 }
 

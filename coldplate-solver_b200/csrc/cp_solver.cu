@@ -110,15 +110,13 @@ struct cp_ctx {
     // smoothed-aggregation hierarchy (pressureSolverType 4); the 2 x 2 one
     // above stays for type 2 and for batches
     bool useSa = false;
-    int saL = 0, saLg = 0;
+    int saL = 0, saLd = 0;                   // levels; first level solved by its V-cycle matrix
     int saNI[kSaMaxLevels] = {}, saNJ[kSaMaxLevels] = {}, saP[kSaMaxLevels] = {};
-    // per level: c[0..8] x y b t pw[0..3] (level 0: x y b t and pw[0..2];
-    // pw only on levels that run grid-wide and have a coarser one)
-    void* saArr[kSaMaxLevels][17] = {};
+    // per level: c[0..8] x y b pw[0..3] (level 0: y, the second CG residual
+    // and pw[0..2]; pw only on levels that have a coarser one)
+    void* saArr[kSaMaxLevels][16] = {};
     void* saDinv0 = nullptr;                 // level-0 inverse diagonal
-    size_t saSmem = 0;                       // k_pcg_sa's dynamic shared memory (bytes)
-    void* saY[9] = {};
-    void* saDense = nullptr;
+    void* saBm[kSaMaxLevels] = {};           // V-cycle matrices of levels [saLd, saL)
     double saOmega = 0.9, saW0 = 2.0 / 3.0, saWc = 0.8;
     unsigned long long* saProf = nullptr;    // per-phase timers when CP_SA_PROFILE is set
     int saReuse = 4;                         // outer iterations between coarse-operator rebuilds
@@ -494,38 +492,30 @@ SaHier<TV> sa_hier(cp_ctx* c) {
     SaHier<TV> H;
     memset(&H, 0, sizeof(H));
     H.L = c->saL;
-    H.Lg = c->saLg;
+    H.Ld = c->saLd;
     H.omega = c->saOmega;
     H.w0 = c->saW0;
     H.wc = c->saWc;
-    H.dense = (TV*)c->saDense;
     H.prof = c->saProf;
     H.r2 = (TV*)c->saArr[0][11];
     H.dinv0 = (TV*)c->saDinv0;
     H.reuse = c->saReuse;
     H.dirty = c->saDirty;
-    for (int q = 0; q < 9; ++q) H.Y[q] = (TV*)c->saY[q];
     for (int l = 0; l < c->saL; ++l) {
         SaLevel<TV>& v = H.lv[l];
+        H.bm[l] = (TV*)c->saBm[l];
         v.nI = c->saNI[l]; v.nJ = c->saNJ[l]; v.P = c->saP[l];
         TV** a = reinterpret_cast<TV**>(c->saArr[l]);
         for (int q = 0; q < 9; ++q) v.c[q] = a[q];
-        v.x = a[9]; v.y = a[10]; v.b = a[11]; v.t = a[12];
-        for (int q = 0; q < 4; ++q) v.pw[q] = a[13 + q];
+        v.x = a[9]; v.y = a[10]; v.b = a[11];
+        for (int q = 0; q < 4; ++q) v.pw[q] = a[12 + q];
     }
     return H;
 }
 
-// dynamic shared memory of k_pcg_sa: the dense set-up workspace, then CTA
-// 0's staged levels (at most kSaSmemBudget bytes)
-constexpr size_t kSaDynSmem = sizeof(double) * (size_t)(kSaDense * 2 * kSaDense + kSaDense);
-constexpr size_t kSaSmemMax = kSaDynSmem > kSaSmemBudget ? kSaDynSmem : kSaSmemBudget;
-static_assert(kSaSmemMax + 4096 <= 227 * 1024, "k_pcg_sa's dynamic shared memory exceeds a block's limit");
-
 // Level sizes of the smoothed aggregation: 3 x 3 aggregates (rounding up)
-// until at most kSaDense unknowns.  Level 0 and the levels above kSaCtaCells
-// unknowns run grid-wide, and so do further levels until the rest fits CTA
-// 0's shared-memory budget.
+// until at most kSaDense unknowns.  From the first coarse level with at most
+// kSaApply unknowns on, the V-cycle is a stored matrix.
 cp_status sa_build(cp_ctx* c) {
     int nI = c->d.M - 1, nJ = c->d.N - 2;
     int L = 0;
@@ -537,20 +527,14 @@ cp_status sa_build(cp_ctx* c) {
         nI = sa_coarse(nI); nJ = sa_coarse(nJ);
     }
     c->saL = L;
-    size_t budget = kSaSmemBudget;
-    if (const char* e = getenv("CP_SA_SMEM_KB")) budget = std::min(budget, (size_t)std::max(atoi(e), 1) * 1024);
-    int Lg = 1;
-    while (Lg < L - 1 && ((long long)c->saNI[Lg] * c->saNJ[Lg] > kSaCtaCells ||
-                          sa_cta_elems(c->saNI, c->saNJ, Lg, L) * c->es > budget))
-        ++Lg;
-    c->saLg = Lg;
-    c->saSmem = std::max(kSaDynSmem, sa_cta_elems(c->saNI, c->saNJ, Lg, L) * c->es);
-    if (c->saSmem > kSaSmemMax) return fail(CP_ERR_BAD_PARAM, "smoothed-aggregation coarsest level too large");
+    int Ld = 1;
+    while ((long long)c->saNI[Ld] * c->saNJ[Ld] > kSaApply) ++Ld;
+    c->saLd = Ld;
     c->saP[0] = c->d.P;
     cp_status s;
-    // level 0: pre-smoothed iterate, corrected iterate, the second CG
-    // residual buffer (its rhs is the CG residual), scratch
-    for (int q = 9; q <= 15; ++q)
+    // level 0: corrected iterate, the second CG residual buffer (its rhs is
+    // the CG residual), prolongation weights
+    for (int q : {10, 11, 12, 13, 14})
         if ((s = dalloc_bytes(c, &c->saArr[0][q], c->nElem * c->es)) != CP_OK) return s;
     if ((s = dalloc_bytes(c, &c->saDinv0, c->nElem * c->es)) != CP_OK) return s;
     if ((s = dalloc(c, &c->saDirty, 1)) != CP_OK) return s;
@@ -561,26 +545,23 @@ cp_status sa_build(cp_ctx* c) {
     for (int l = 1; l < L; ++l) {
         c->saP[l] = ((c->saNJ[l] + 2 + 31) / 32) * 32;
         const size_t ne = (size_t)(c->saNI[l] + 2) * c->saP[l];
-        const int nq = (l < Lg && l < L - 1) ? 17 : 13;
-        for (int q = 0; q < nq; ++q)
+        for (int q = 0; q < (l < L - 1 ? 16 : 12); ++q)
             if ((s = dalloc_bytes(c, &c->saArr[l][q], ne * c->es)) != CP_OK) return s;
+        if (l >= Ld) {
+            const size_t n = (size_t)c->saNI[l] * c->saNJ[l];
+            if ((s = dalloc_bytes(c, &c->saBm[l], n * c->saNI[l] * c->saP[l] * c->es)) != CP_OK) return s;
+        }
     }
-    for (int q = 0; q < 9; ++q)
-        if ((s = dalloc_bytes(c, &c->saY[q], c->nElem * c->es)) != CP_OK) return s;
-    if ((s = dalloc_bytes(c, &c->saDense, (size_t)kSaDense * kSaDense * c->es)) != CP_OK) return s;
     if (const char* e = getenv("CP_SA_OMEGA")) c->saOmega = atof(e);
     if (const char* e = getenv("CP_SA_W0")) c->saW0 = atof(e);
     if (const char* e = getenv("CP_SA_WC")) c->saWc = atof(e);
     if (const char* e = getenv("CP_SA_REUSE")) c->saReuse = std::max(atoi(e), 1);
     if (getenv("CP_SA_PROFILE") && (s = dalloc(c, &c->saProf, (size_t)SA_P_COUNT)) != CP_OK) return s;
     int nb = 0;
-    if (c->prm.precision == CP_PREC_MIXED) {
-        cudaFuncSetAttribute(k_pcg_sa<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSaSmemMax);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pcg_sa<float>, kMgThreads, c->saSmem);
-    } else {
-        cudaFuncSetAttribute(k_pcg_sa<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSaSmemMax);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pcg_sa<double>, kMgThreads, c->saSmem);
-    }
+    if (c->prm.precision == CP_PREC_MIXED)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pcg_sa<float>, kMgThreads, kSaSmem);
+    else
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pcg_sa<double>, kMgThreads, kSaSmem);
     if (nb < 1) return fail(CP_ERR_CUDA, "smoothed-aggregation PCG kernel does not fit on an SM");
     return CP_OK;
 }
@@ -629,7 +610,7 @@ cp_status enqueue_pressure(cp_ctx* c, EvRec* rec = nullptr) {
     REC_BEGIN(rec, CP_K_PCG);
     if (c->useSa) {
         SaHier<TV> H = sa_hier<TV>(c);
-        CK(launch_coop_cfg(k_pcg_sa<TV>, c->gMg, kMgThreads, c->saSmem, c->stream, c->k, c->st,
+        CK(launch_coop_cfg(k_pcg_sa<TV>, c->gMg, kMgThreads, kSaSmem, c->stream, c->k, c->st,
                            (const double*)c->dE, (const double*)c->dN, B, H, c->pStar, c->partP, c->barP));
     } else if (c->useMg) {
         MgHier<TV> H = mg_hier<TV>(c);
@@ -945,7 +926,7 @@ cp_status cp_create(const cp_params* prm, cp_ctx** out) {
     if (c->useSa && (s = sa_build(c)) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->partJ, (size_t)4 * c->gJac)) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->partM, (size_t)4 * c->nbMass)) != CP_OK) return bail(s);
-    if ((s = dalloc(c, &c->partP, (size_t)3 * std::max(c->gPcg, c->gMg))) != CP_OK) return bail(s);
+    if ((s = dalloc(c, &c->partP, (size_t)4 * std::max(c->gPcg, c->gMg))) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->barJ, 1)) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->barP, 1)) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->st, 1)) != CP_OK) return bail(s);
@@ -972,11 +953,11 @@ cp_status cp_destroy(cp_ctx* c) {
         // summed over the context's life (block 0's clock after each barrier)
         unsigned long long t[SA_P_COUNT];
         if (cudaMemcpy(t, c->saProf, sizeof t, cudaMemcpyDeviceToHost) == cudaSuccess) {
-            fprintf(stderr, "CP_SA_PROFILE ms: setup %.3f galerkin %.3f matvec %.3f update %.3f cta %.3f", t[SA_P_SETUP] * 1e-6,
-                    t[SA_P_GALERKIN] * 1e-6, t[SA_P_MATVEC] * 1e-6, t[SA_P_UPDATE] * 1e-6, t[SA_P_CTA] * 1e-6);
-            for (int l = 0; l < c->saLg; ++l) fprintf(stderr, " down%d %.3f", l, t[SA_P_DOWN + l] * 1e-6);
-            for (int l = 0; l < c->saLg; ++l) fprintf(stderr, " up%d %.3f", l, t[SA_P_UP + l] * 1e-6);
-            fprintf(stderr, " levels %d grid %d\n", c->saL, c->saLg);
+            fprintf(stderr, "CP_SA_PROFILE ms: setup %.3f galerkin %.3f matvec %.3f update %.3f dense %.3f", t[SA_P_SETUP] * 1e-6,
+                    t[SA_P_GALERKIN] * 1e-6, t[SA_P_MATVEC] * 1e-6, t[SA_P_UPDATE] * 1e-6, t[SA_P_DENSE] * 1e-6);
+            for (int l = 1; l < c->saLd; ++l) fprintf(stderr, " down%d %.3f", l, t[SA_P_DOWN + l] * 1e-6);
+            for (int l = 0; l < c->saLd; ++l) fprintf(stderr, " up%d %.3f", l, t[SA_P_UP + l] * 1e-6);
+            fprintf(stderr, " levels %d grid %d\n", c->saL, c->saLd);
         }
     }
     if (c->graph) cudaGraphExecDestroy(c->graph);
@@ -1263,7 +1244,7 @@ cp_status adjoint_pcg(cp_ctx* c, const KParams& k, const double* dE, const doubl
         // flags stale at the start)
         H.dirty = c->saDirtyAdj;
         H.reuse = 0;
-        CK(launch_coop_cfg(k_pcg_sa<TV>, c->gMg, kMgThreads, c->saSmem, c->stream, k, c->adjSt, dE, dN, B, H, out,
+        CK(launch_coop_cfg(k_pcg_sa<TV>, c->gMg, kMgThreads, kSaSmem, c->stream, k, c->adjSt, dE, dN, B, H, out,
                            c->adjPart, c->adjBar));
     } else if (c->useMg) {
         MgHier<TV> H = mg_hier<TV>(c);
@@ -1911,7 +1892,6 @@ struct cp_batch {
     // team mode (every field runs smoothed aggregation): k_batch_team
     bool teamMode = false;
     int team = 4, nTeams = 0;    // CTAs per team, teams
-    size_t teamSmem = 0;         // dynamic shared memory (the largest field's k_pcg_sa staging)
     int* dOrder = nullptr;       // queue order, largest field first
     unsigned* dTbar = nullptr;   // [grid * kTeamStride] team barrier counters
     int* dQueue = nullptr;       // [1 + 2 grid]
@@ -2023,7 +2003,7 @@ cp_status batch_launch_team(cp_batch* b, int nOuter) {
     CK(cudaMemsetAsync(b->dTbar, 0, (size_t)b->grid * kTeamStride * sizeof(unsigned), b->stream));
     CK(cudaMemsetAsync(b->dQueue, 0, (size_t)(1 + 2 * b->grid) * sizeof(int), b->stream));
     CK(cudaMemsetAsync(b->dRunning, 0, sizeof(int), b->stream));
-    CK(launch_coop_cfg(k_batch_team<TC, Mixed>, b->grid, kBatchThreads, b->teamSmem, b->stream, a,
+    CK(launch_coop_cfg(k_batch_team<TC, Mixed>, b->grid, kBatchThreads, kSaSmem, b->stream, a,
                        (const BFieldSa<TC>*)b->dF));
     return CP_OK;
 }
@@ -2238,18 +2218,10 @@ cp_status cp_batch_create(cp_ctx* const* fields, int n, cp_batch** out) {
     // one block per SM: the kernel must fit with its shared-memory workspace
     int nb = 0;
     if (b->teamMode) {
-        for (cp_ctx* c : b->f) b->teamSmem = std::max(b->teamSmem, c->saSmem);
-        if (b->mixed) {
-            cudaFuncSetAttribute(k_batch_team<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)b->teamSmem);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_team<float, true>, kBatchThreads,
-                                                          b->teamSmem);
-        } else {
-            cudaFuncSetAttribute(k_batch_team<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)b->teamSmem);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_team<double, false>, kBatchThreads,
-                                                          b->teamSmem);
-        }
+        if (b->mixed)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_team<float, true>, kBatchThreads, kSaSmem);
+        else
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_team<double, false>, kBatchThreads, kSaSmem);
     } else if (b->mixed) {
         cudaFuncSetAttribute(k_batch<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchDynSmem);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch<float, true>, kBatchThreads, kBatchDynSmem);
