@@ -693,11 +693,8 @@ __device__ __forceinline__ bool team_outer(const Team& T, unsigned& target, cons
     // ---- k_jacobi: U sweeps, V sweeps, scatter with clamps, BCs on u*, v*
     {
         int curU = -1, curV = -1, itU = 0, itV = 0;
-        if (!jacobi_component<TC, Mixed, true>(k, f.U, f.u, f.xU0, f.xU1, f.partJ, T, target, curU, itU))
-            return false;
-        if (!jacobi_component<TC, Mixed, false>(k, f.V, f.v, f.xV0, f.xV1, f.partJ + 2 * T.size, T, target, curV,
-                                                itV))
-            return false;
+        if (!jacobi_component<TC, Mixed, true>(k, f.U, f.u, f.xU0, f.xU1, f.partJ, T, target, curU, itU)) return false;
+        if (!jacobi_component<TC, Mixed, false>(k, f.V, f.v, f.xV0, f.xV1, f.partJ, T, target, curV, itV)) return false;
         double mu = jacobi_scatter<TC, Mixed, true>(k, f.u, curU < 0 ? nullptr : (curU ? f.xU1 : f.xU0), f.uStar,
                                                     maxVel, tid, nth);
         double mv = jacobi_scatter<TC, Mixed, false>(k, f.v, curV < 0 ? nullptr : (curV ? f.xV1 : f.xV0), f.vStar,

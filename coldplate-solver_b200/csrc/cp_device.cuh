@@ -224,6 +224,7 @@ __device__ __forceinline__ bool team_sync(const Team& T, unsigned& target) {
 // rewritten only after every CTA has passed a later barrier.  sm: kReduceSm
 // doubles, written by team_reduce alone.
 constexpr int kReduceSm = 68;
+constexpr int kReduceLoads = 5;   // partials a lane has in flight (148 CTAs: all of them)
 template <int NV>
 __device__ __forceinline__ bool team_reduce(const Team& T, unsigned& target, double (&v)[NV], double* part,
                                             double* sm) {
@@ -240,22 +241,34 @@ __device__ __forceinline__ bool team_reduce(const Team& T, unsigned& target, dou
         double* slot = part + ((target / (unsigned)T.size) & 1u) * 2 * T.size;
         double t[NV];
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            t[k] = warp_sum(lane < nw ? sm[k * 32 + lane] : 0.0);
-            if (lane == 0) __stcg(slot + NV * T.rank + k, t[k]);
-        }
+        for (int k = 0; k < NV; ++k) t[k] = lane < nw ? sm[k * 32 + lane] : 0.0;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) t[k] = warp_sum(t[k]);
+        if (lane == 0)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) __stcg(slot + NV * T.rank + k, t[k]);
         int ok = 1;
         if (lane == 0) ok = barrier_arrive_wait(T.bar, target, T.err) ? 1 : 0;
         __syncwarp();
         ok = __shfl_sync(0xffffffffu, ok, 0);
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            t[k] = 0.0;
-            if (ok)
-                for (int b = lane; b < T.size; b += 32) t[k] += __ldcg(slot + NV * b + k);
-            t[k] = warp_sum(t[k]);
-            if (lane == 0) sm[64 + k] = t[k];
+        for (int k = 0; k < NV; ++k) t[k] = 0.0;
+        for (int b0 = lane; ok && b0 - lane < T.size; b0 += 32 * kReduceLoads) {
+            double q[kReduceLoads][NV];
+#pragma unroll
+            for (int u = 0; u < kReduceLoads; ++u)
+#pragma unroll
+                for (int k = 0; k < NV; ++k) q[u][k] = b0 + 32 * u < T.size ? __ldcg(slot + NV * (b0 + 32 * u) + k) : 0.0;
+#pragma unroll
+            for (int u = 0; u < kReduceLoads; ++u)
+#pragma unroll
+                for (int k = 0; k < NV; ++k) t[k] += q[u][k];
         }
+#pragma unroll
+        for (int k = 0; k < NV; ++k) t[k] = warp_sum(t[k]);
+        if (lane == 0)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) sm[64 + k] = t[k];
         if (lane == 0) sm[66] = (double)ok;
     }
     __syncthreads();

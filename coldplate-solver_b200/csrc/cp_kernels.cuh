@@ -33,6 +33,9 @@
 
 namespace cp {
 
+constexpr int kJacThreads = 512;      // sweeps of both components: one CTA an SM
+constexpr int kJacSegThreads = 256;   // one component after the other: three CTAs an SM
+
 // ------------------------------------------------------------------ systems
 template <typename TC>
 struct MomSys {
@@ -248,18 +251,174 @@ __global__ void __launch_bounds__(256, 4) k_assemble(KParams k, const Status* st
 }
 
 // ------------------------------------------------------------------ Jacobi
-// One component's sweeps.  Each thread handles two rows per loop trip with
-// all loads issued before the arithmetic (memory-level parallelism); the
-// sum of r^2 is reduced per sweep, one grid barrier per sweep.  Returns the
-// buffer index holding the result (-1: the initial iterate) and the sweep
-// count, or false if a barrier gave up.
+// Jacobi sweeps x+ = x + (b - A x) / aP of the U and the V system (they are
+// independent: V assembles from u, v, not from u*).  Each component stops
+// after the first sweep whose pre-update sum of r^2 is below tol^2 n, or after
+// maxMomentumIter sweeps (jacobi_solver.cpp:44-67).
+//
+// A sweep is short (8 words an unknown from the L2), so the barrier and the
+// sum behind it count: both components sweep between the same two barriers
+// while both run, and the sums ride on the barrier (team_reduce).  The sweeps
+// of an outer iteration took 103 us one after the other and take 72 together
+// at 253 x 127 (double, 21 sweeps of one component), 163 and 131 at 811 x 389
+// (float, 30), 1.04 and 0.93 ms at 2048 x 1024 (double, 33).
+// A warp takes a run of rows of a strip of 30 V columns: the next row's
+// coefficients are in flight while it works on one, the iterate's rows stay in
+// registers and its horizontal neighbours come by shuffles (lanes 0 and 31
+// only supply them).  V = 16 bytes where the grid has more rows of strips than
+// warps; otherwise the smallest that gives every warp at most one row, which
+// puts all of a sweep's loads in flight at once.
+template <typename TC, bool Mixed, int V>
+__device__ __forceinline__ double jacobi_run(const Dims& d, const MomSys<TC>& S, const double* field, const TC* xc,
+                                             TC* __restrict__ xn, int j1, int s, int i0, int i1) {
+    const int lane = threadIdx.x & 31;
+    const int g = 30 * s - 1 + lane, j0 = g * V;
+    const bool act = g >= 0 && g < j1 / V + 1, own = act && lane >= 1 && lane <= 30;
+    struct Row {
+        VecN<TC, V> aP, aE, aW, aN, aS, b;
+    };
+    auto ldr = [&](int i, bool on) {
+        Row r;
+        if (on) {
+            const size_t q = at(d, i, j0);
+            r = Row{ldv<V>(S.aP + q), ldv<V>(S.aE + q), ldv<V>(S.aW + q), ldv<V>(S.aN + q), ldv<V>(S.aS + q), ldv<V>(S.b + q)};
+        } else {
+            r = Row{zerov<TC, V>(), zerov<TC, V>(), zerov<TC, V>(), zerov<TC, V>(), zerov<TC, V>(), zerov<TC, V>()};
+        }
+        return r;
+    };
+    // the iterate (the current field, or zero in the mixed form, before the
+    // first sweep); couplings to anything outside the unknowns are zero
+    auto ldx = [&](int i, bool on) -> VecN<TC, V> {
+        if (!on) return zerov<TC, V>();
+        if (xc) return ldv<V>(xc + at(d, i, j0));
+        if constexpr (Mixed) return zerov<TC, V>();
+        else return ldv<V>(field + at(d, i, j0));
+    };
+    VecN<TC, V> xS = ldx(i0 - 1, own), xP = ldx(i0, act), xN = ldx(i0 + 1, act);
+    Row cur = ldr(i0, own);
+    double acc = 0.0;
+#pragma unroll 1
+    for (int i = i0; i <= i1; ++i) {
+        const bool more = i < i1;
+        const VecN<TC, V> xF = ldx(i + 2, act && more);
+        const Row nxt = ldr(i + 1, own && more);
+        const TC xw = from_west(xP.v[V - 1]), xe = from_east(xP.v[0]);
+        VecN<TC, V> o;
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+            const int j = j0 + q;
+            const bool in = own && j >= 1 && j <= j1;
+            const TC W = q ? xP.v[q ? q - 1 : 0] : xw, E = q < V - 1 ? xP.v[q < V - 1 ? q + 1 : 0] : xe;
+            // S, W, P, E, N order of the reference's CSR rows
+            TC Ax = (TC)0;
+            Ax += (-cur.aS.v[q]) * xS.v[q];
+            Ax += (-cur.aW.v[q]) * W;
+            Ax += cur.aP.v[q] * xP.v[q];
+            Ax += (-cur.aE.v[q]) * E;
+            Ax += (-cur.aN.v[q]) * xN.v[q];
+            const TC r = cur.b.v[q] - Ax;
+            const TC dg = in ? cur.aP.v[q] : (TC)1;
+            o.v[q] = in ? (TC)(xP.v[q] + r / dg) : (TC)0;
+            if (in) acc += (double)r * (double)r;
+        }
+        if (own) stv(xn + at(d, i, j0), o);
+        xS = xP;
+        xP = xN;
+        xN = xF;
+        cur = nxt;
+    }
+    return acc;
+}
+
+// One component of a sweep: its strips and rows, and the runs they are cut into
+struct JacSplit {
+    int S, R, n, rows;
+    __device__ __forceinline__ JacSplit(int V, int i1, int j1, int nw, int both) {
+        S = (j1 / V + 30) / 30;
+        rows = i1;
+        R = max(1, (i1 * S * both + nw - 1) / nw);
+        n = S * ((i1 + R - 1) / R);
+    }
+};
+
+template <typename TC, bool Mixed, int V>
+__device__ __forceinline__ void jacobi_pass(const KParams& k, const MomSys<TC>& U, const MomSys<TC>& W, const double* u,
+                                            const double* v, const TC* xUc, TC* xUn, const TC* xVc, TC* xVn,
+                                            bool doU, bool doV, const Team& T, double (&acc)[2]) {
+    const int nw = T.nth() >> 5, wid = threadIdx.x >> 5;
+    int iU, jU, iV, jV;
+    mom_range<true>(k.d, iU, jU);
+    mom_range<false>(k.d, iV, jV);
+    const int both = doU && doV ? 2 : 1;
+    const JacSplit sU(V, iU, jU, nw, both), sV(V, iV, jV, nw, both);
+    const int nU = doU ? sU.n : 0, n = nU + (doV ? sV.n : 0);
+    // with fewer runs than warps, spread over the CTAs
+    for (int c = n < nw ? wid * T.size + T.rank : T.rank * (int)(blockDim.x >> 5) + wid; c < n; c += nw) {
+        if (c < nU) {
+            const int i0 = 1 + c / sU.S * sU.R;
+            acc[0] += jacobi_run<TC, Mixed, V>(k.d, U, u, xUc, xUn, jU, c % sU.S, i0, min(iU, i0 + sU.R - 1));
+        } else {
+            const int e = c - nU, i0 = 1 + e / sV.S * sV.R;
+            acc[1] += jacobi_run<TC, Mixed, V>(k.d, W, v, xVc, xVn, jV, e % sV.S, i0, min(iV, i0 + sV.R - 1));
+        }
+    }
+}
+
+// The sweeps of both components (or of one); cur: the buffer that holds the
+// result (-1: the initial iterate), its: the sweeps.  part: 4 doubles a CTA.
+// Returns false if a barrier gave up.
+template <typename TC, bool Mixed>
+__device__ __forceinline__ bool jacobi_sweeps(const KParams& k, const MomSys<TC>& U, const MomSys<TC>& W, const double* u,
+                                              const double* v, TC* xU0, TC* xU1, TC* xV0, TC* xV1, bool doU, bool doV,
+                                              double* part, const Team& T, unsigned& target, int& curU, int& curV,
+                                              int& itU, int& itV) {
+    __shared__ double sm[kReduceSm];
+    const int nw = T.nth() >> 5;
+    const double lim = k.momTol * k.momTol, limU = lim * (double)k.nU, limV = lim * (double)k.nV;
+    curU = curV = -1;
+    itU = itV = 0;
+    bool onU = doU && k.maxMom > 0, onV = doV && k.maxMom > 0;
+    while (onU || onV) {
+        const TC* xUc = curU < 0 ? nullptr : (curU ? xU1 : xU0);
+        const TC* xVc = curV < 0 ? nullptr : (curV ? xV1 : xV0);
+        TC* xUn = curU == 0 ? xU1 : xU0;
+        TC* xVn = curV == 0 ? xV1 : xV0;
+        double acc[2] = {0.0, 0.0};
+        // rows of strips at V = 1 of the components that still sweep
+        const int rows = (onU ? k.d.M - 1 : 0) + (onV ? k.d.M - 2 : 0);
+        if ((k.d.N + 30) / 30 * rows <= nw)
+            jacobi_pass<TC, Mixed, 1>(k, U, W, u, v, xUc, xUn, xVc, xVn, onU, onV, T, acc);
+        else if (sizeof(TC) == 4 && (k.d.N / 2 + 30) / 30 * rows <= nw)
+            jacobi_pass<TC, Mixed, sizeof(TC) == 4 ? 2 : 1>(k, U, W, u, v, xUc, xUn, xVc, xVn, onU, onV, T, acc);
+        else
+            jacobi_pass<TC, Mixed, Vec16<TC>::n>(k, U, W, u, v, xUc, xUn, xVc, xVn, onU, onV, T, acc);
+        if (!team_reduce(T, target, acc, part, sm)) return false;
+        if (onU) {
+            curU = curU == 0 ? 1 : 0;
+            onU = ++itU < k.maxMom && !(acc[0] < limU);
+        }
+        if (onV) {
+            curV = curV == 0 ? 1 : 0;
+            onV = ++itV < k.maxMom && !(acc[1] < limV);
+        }
+    }
+    return true;
+}
+
+// The sweeps of one component on row segments (32 lane groups of 16 bytes),
+// one segment a warp and trip.  Used where one component's system stays in the
+// L2 and both together do not (host: jacobi_sequential), and in the batched
+// kernel, whose fields share the L2: there the sweeps of U and then V beat
+// those of both at once (34 sweeps at 2048 x 1024 in float: 0.42 against
+// 0.58 ms; 24 batched fields: 155 against 172 ms), and more warps with fewer
+// registers beat the prefetch (0.42 against 0.49 ms).
 template <typename TC, bool Mixed, bool IsU>
 __device__ __forceinline__ bool jacobi_component(const KParams& k, const MomSys<TC>& S, const double* field,
                                                  TC* x0, TC* x1, double* part, const Team& T, unsigned& target,
                                                  int& cur, int& its) {
-    __shared__ double sm[32];
+    __shared__ double sm[kReduceSm];
     const Dims d = k.d;
-    const int G = T.size;
     int i1, j1;
     mom_range<IsU>(d, i1, j1);
     const int n = i1 * j1;
@@ -324,15 +483,10 @@ __device__ __forceinline__ bool jacobi_component(const KParams& k, const MomSys<
             }
             if (act) st16(xn + c, o);
         });
-        block_sum<1>(acc, sm);
-        double* slot = part + (size_t)(s & 1) * G;
-        if (threadIdx.x == 0) slot[T.rank] = acc[0];
-        if (!team_sync(T, target)) return false;
-        double tot[1];
-        sum_partials<1>(slot, G, 1, tot, sm);
+        if (!team_reduce(T, target, acc, part, sm)) return false;
         cur = nxt;
         its = s + 1;
-        if (tot[0] < lim) break;
+        if (acc[0] < lim) break;
     }
     return true;
 }
@@ -358,18 +512,14 @@ __device__ __forceinline__ double jacobi_scatter(const KParams& k, const double*
     return m;
 }
 
-// Jacobi sweeps x+ = x + (b - A x) / aP of the U system, then of the V
-// system (they are independent: V assembles from u, v, not from u*).  Each
-// component stops after the first sweep whose pre-update sum of r^2 is
-// below tol^2 n, or after maxMomentumIter sweeps (jacobi_solver.cpp:44-67).
-// Running the components one after the other keeps one component's system
-// resident in L2.  Then the scatter with clamps and the BCs on u*, v*.
 struct JacobiOut {
     double *uStar, *vStar;
 };
 
-template <typename TC, bool Mixed>
-__global__ void __launch_bounds__(256) k_jacobi(KParams k, Status* st, MomSys<TC> U, MomSys<TC> V,
+// The sweeps (Seq: one component after the other), then the scatter with
+// clamps and the BCs on u*, v*
+template <typename TC, bool Mixed, bool Seq>
+__global__ void __launch_bounds__(Seq ? kJacSegThreads : kJacThreads, Seq ? 3 : 1) k_jacobi(KParams k, Status* st, MomSys<TC> U, MomSys<TC> V,
                                                 const double* u, const double* v, TC* xU0, TC* xU1, TC* xV0,
                                                 TC* xV1, JacobiOut out, const double* gamma, double* part,
                                                 unsigned* bar, int doU, int doV, int applyBC) {
@@ -381,10 +531,13 @@ __global__ void __launch_bounds__(256) k_jacobi(KParams k, Status* st, MomSys<TC
     unsigned target = 0;
     const Team T = grid_team(bar, &st->err);
     int curU = -1, curV = -1, itU = 0, itV = 0;
-    if (doU && !jacobi_component<TC, Mixed, true>(k, U, u, xU0, xU1, part, T, target, curU, itU)) return;
-    // V uses its own partial slots: blocks may still read U's last sums
-    if (doV && !jacobi_component<TC, Mixed, false>(k, V, v, xV0, xV1, part + 2 * G, T, target, curV, itV))
-        return;
+    if constexpr (Seq) {
+        if (doU && !jacobi_component<TC, Mixed, true>(k, U, u, xU0, xU1, part, T, target, curU, itU)) return;
+        if (doV && !jacobi_component<TC, Mixed, false>(k, V, v, xV0, xV1, part, T, target, curV, itV)) return;
+    } else {
+        if (!jacobi_sweeps<TC, Mixed>(k, U, V, u, v, xU0, xU1, xV0, xV1, doU, doV, part, T, target, curU, curV, itU, itV))
+            return;
+    }
     double mu = 0.0, mv = 0.0;
     if (doU) mu = jacobi_scatter<TC, Mixed, true>(k, u, curU < 0 ? nullptr : (curU ? xU1 : xU0), out.uStar, maxVel, tid, nth);
     if (doV) mv = jacobi_scatter<TC, Mixed, false>(k, v, curV < 0 ? nullptr : (curV ? xV1 : xV0), out.vStar, maxVel, tid, nth);

@@ -88,6 +88,7 @@ struct cp_ctx {
     double* hist = nullptr;
     int histCap = 0;
     double* dpWin = nullptr;
+    bool jacSeq = false;               // sweeps of U, then of V (jacobi_sequential)
     int gJac = 0, gPcg = 0, gElem = 0, nbMass = 0;
     // multigrid hierarchy (pressureSolverType 2 / 4)
     bool useMg = false;
@@ -201,6 +202,17 @@ cp_status validate(const cp_params* p) {
     if (p->usePressureDropConvergence && p->dpConvergenceWindow <= 0)
         return fail(CP_ERR_BAD_PARAM, "dpConvergenceWindow must be > 0");
     return CP_OK;
+}
+
+// Whether the Jacobi kernel sweeps U to its end and then V.  A component's
+// sweeps read eight arrays; where those of one component stay in the 126 MB L2
+// and those of both do not, one at a time is faster (2048 x 1024 in float,
+// 67 MB each: 0.42 against 0.58 ms).  Where both fit (131 against 163 us at
+// 811 x 389) and where not even one does (2048 x 1024 in double, 134 MB each:
+// 0.93 against 1.04 ms) both at once are, for their fewer barriers.
+bool jacobi_sequential(const cp_ctx* c) {
+    const size_t one = 8 * c->nElem * c->es, l2 = 100u << 20;
+    return one <= l2 && 2 * one > l2;
 }
 
 void fill_kparams(cp_ctx* c) {
@@ -592,7 +604,8 @@ cp_status enqueue_momentum(cp_ctx* c, int doU, int doV, int applyBC, EvRec* rec 
     CK(cudaMemsetAsync(c->barJ, 0, sizeof(unsigned), c->stream));
     JacobiOut out{c->uStar, c->vStar};
     REC_BEGIN(rec, CP_K_JACOBI);
-    CK(launch_coop(k_jacobi<TC, Mixed>, c->gJac, c->stream, c->k, c->st, U, V, (const double*)c->u,
+    CK(launch_coop_cfg(c->jacSeq ? k_jacobi<TC, Mixed, true> : k_jacobi<TC, Mixed, false>, c->gJac,
+                   c->jacSeq ? kJacSegThreads : kJacThreads, 0, c->stream, c->k, c->st, U, V, (const double*)c->u,
                    (const double*)c->v, (TC*)c->xb[0], (TC*)c->xb[1], (TC*)c->xb[2], (TC*)c->xb[3], out,
                    (const double*)c->gamma, c->partJ, c->barJ, doU, doV, applyBC));
     REC_END(rec);
@@ -896,22 +909,20 @@ cp_status cp_create(const cp_params* prm, cp_ctx** out) {
         if ((s = dalloc_bytes(c, &x, c->nElem * c->es)) != CP_OK) return bail(s);
     for (auto& x : c->pcg)
         if ((s = dalloc_bytes(c, &x, c->nElem * c->es)) != CP_OK) return bail(s);
+    c->jacSeq = jacobi_sequential(c);
     // cooperative grids: every block must be resident
     int nbJ = 0, nbP = 0;
     if (c->prm.precision == CP_PREC_MIXED) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<float, true>, kThreads, 0);
+        if (c->jacSeq) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<float, true, true>, kJacSegThreads, 0);
+        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<float, true, false>, kJacThreads, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbP, k_pcg<float>, kThreads, 0);
     } else {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<double, false>, kThreads, 0);
+        if (c->jacSeq) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<double, false, true>, kJacSegThreads, 0);
+        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<double, false, false>, kJacThreads, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbP, k_pcg<double>, kThreads, 0);
     }
     if (nbJ < 1 || nbP < 1) return bail(fail(CP_ERR_CUDA, "cooperative kernels do not fit on an SM"));
-    // as many Jacobi CTAs per SM as fit (float: 3 of 256 threads, 12 % faster
-    // sweeps at 2048 x 1024 than 2; double: 2), at most 4; CP_JACOBI_CTAS
-    // caps it lower
-    int jacCtas = 4;
-    if (const char* e = getenv("CP_JACOBI_CTAS")) jacCtas = std::max(atoi(e), 1);
-    c->gJac = c->numSMs * std::min(nbJ, jacCtas);
+    c->gJac = c->numSMs * (c->jacSeq ? std::min(nbJ, 3) : 1);
     c->gPcg = c->numSMs * std::min(nbP, 4);
     c->gElem = c->numSMs * 4;
     c->nbMass = c->numSMs * 4;
