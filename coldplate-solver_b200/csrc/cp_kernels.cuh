@@ -612,135 +612,6 @@ __global__ void k_mass(KParams k, const Status* st, const double* u, const doubl
                   part + (size_t)blockIdx.x * 4);
 }
 
-// ------------------------------------------------------------------ PCG
-// Jacobi-preconditioned CG on the pressure correction (pressure_solver.cpp:121-184):
-//   unknowns (i, j) in [1, M-1] x [1, N-2]; p'(:, N-1) = 0;
-//   aE = rho dE(i,j) hy, aW = rho dE(i,j-1) hy (j > 1), aN = rho dN(i,j) hx
-//   (i < M-1), aS = rho dN(i-1,j) hx (i > 1); aP = aE+aW+aN+aS (1 if < 1e-20).
-// Matrix-free: fE(i,j) holds the east-face coefficient (zero at j = 0) and
-// fN(i,j) the north-face one (zero at rows 0 and M-1); direction vectors are
-// zero outside the unknowns, so the stencil needs no branches.
-// Per iteration two grid barriers:
-//   A: p_new = z + beta p_old (recomputed at the 4 neighbours from r, d,
-//      p_old; written to the other buffer), Ap = A p_new, partial p.Ap
-//   B: x += alpha p_new, r -= alpha Ap, partials r.r and r.z
-// The reference's early exits are kept: |p.Ap| < 1e-20 and sqrt(r.r) < pTol,
-// and the returned count is the loop index at exit (maxPressureIter if none).
-template <typename TV>
-__device__ __forceinline__ TV pcg_dir(const TV* r, const TV* dd, const TV* pold, size_t c, double beta,
-                                      bool first) {
-    const TV z = r[c] / dd[c];
-    return first ? z : (TV)(z + (TV)beta * pold[c]);
-}
-
-template <typename TV>
-__global__ void __launch_bounds__(256) k_pcg(KParams k, Status* st, const double* dE, const double* dN,
-                                             PcgBufs<TV> B, double* pStar, double* part, unsigned* bar) {
-    if (st->done) return;
-    __shared__ double sm[96];
-    const Dims d = k.d;
-    const int M = d.M, N = d.N, w = N - 2;
-    const int n = (M - 1) * w;
-    const int G = gridDim.x;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = G * blockDim.x;
-    const double rho = k.rho, hx = k.hx, hy = k.hy;
-    unsigned target = 0;
-    double* partA = part;           // [G]     p.Ap
-    double* partB = part + G;       // [G][2]  r.r, r.z
-    // init: faces, diagonal, x = 0, r = b (A 0 = 0), partial r.z
-    double acc0[1] = {0.0};
-    for (int t = tid; t < n; t += nth) {
-        const int i = 1 + t / w, j = 1 + t % w;
-        const size_t c = at(d, i, j);
-        const double aE = rho * dE[c] * hy;
-        const double aW = (j > 1) ? rho * dE[c - 1] * hy : 0.0;
-        const double aN = (i < M - 1) ? rho * dN[c] * hx : 0.0;
-        const double aS = (i > 1) ? rho * dN[c - d.P] * hx : 0.0;
-        double aP = aE + aW + aN + aS;
-        if (aP < 1e-20) aP = 1.0;
-        B.fE[c] = (TV)aE;
-        if (i < M - 1) B.fN[c] = (TV)aN;
-        B.d[c] = (TV)aP;
-        B.x[c] = (TV)0;
-        const TV r = B.rhs[c];
-        B.r[c] = r;
-        acc0[0] += (double)r * (double)(r / (TV)aP);
-    }
-    block_sum<1>(acc0, sm);
-    if (threadIdx.x == 0) partB[2 * blockIdx.x + 1] = acc0[0];
-    target += G;
-    if (!grid_barrier(bar, target, &st->err)) return;
-    double tot1[1];
-    {
-        double t2[2];
-        sum_partials<2>(partB, G, 2, t2, sm);
-        tot1[0] = t2[1];
-    }
-    double rz = tot1[0];
-    double beta = 0.0;
-    int it = 0;
-    TV* pbuf[2] = {B.pa, B.pb};
-    for (; it < k.maxP; ++it) {
-        const bool first = (it == 0);
-        const TV* pold = pbuf[(it + 1) & 1];
-        TV* pnew = pbuf[it & 1];
-        double accA[1] = {0.0};
-        for (int t = tid; t < n; t += nth) {
-            const int i = 1 + t / w, j = 1 + t % w;
-            const size_t c = at(d, i, j);
-            const TV pc = pcg_dir(B.r, B.d, pold, c, beta, first);
-            const TV pS = (i > 1) ? pcg_dir(B.r, B.d, pold, c - d.P, beta, first) : (TV)0;
-            const TV pW = (j > 1) ? pcg_dir(B.r, B.d, pold, c - 1, beta, first) : (TV)0;
-            const TV pE = (j < w) ? pcg_dir(B.r, B.d, pold, c + 1, beta, first) : (TV)0;
-            const TV pN = (i < M - 1) ? pcg_dir(B.r, B.d, pold, c + d.P, beta, first) : (TV)0;
-            TV ap = (TV)0;
-            ap += (-B.fN[c - d.P]) * pS;
-            ap += (-B.fE[c - 1]) * pW;
-            ap += B.d[c] * pc;
-            ap += (-B.fE[c]) * pE;
-            ap += (-B.fN[c]) * pN;
-            pnew[c] = pc;
-            B.Ap[c] = ap;
-            accA[0] += (double)pc * (double)ap;
-        }
-        block_sum<1>(accA, sm);
-        if (threadIdx.x == 0) partA[blockIdx.x] = accA[0];
-        target += G;
-        if (!grid_barrier(bar, target, &st->err)) return;
-        double pAp[1];
-        sum_partials<1>(partA, G, 1, pAp, sm);
-        if (fabs(pAp[0]) < 1e-20) break;
-        const double alpha = rz / pAp[0];
-        double accB[2] = {0.0, 0.0};
-        for (int t = tid; t < n; t += nth) {
-            const int i = 1 + t / w, j = 1 + t % w;
-            const size_t c = at(d, i, j);
-            const TV pc = pnew[c];
-            B.x[c] = B.x[c] + (TV)alpha * pc;
-            const TV r = B.r[c] - (TV)alpha * B.Ap[c];
-            B.r[c] = r;
-            accB[0] += (double)r * (double)r;
-            accB[1] += (double)r * (double)(r / B.d[c]);
-        }
-        block_sum<2>(accB, sm);
-        if (threadIdx.x == 0) { partB[2 * blockIdx.x] = accB[0]; partB[2 * blockIdx.x + 1] = accB[1]; }
-        target += G;
-        if (!grid_barrier(bar, target, &st->err)) return;
-        double tB[2];
-        sum_partials<2>(partB, G, 2, tB, sm);
-        if (sqrt(tB[0]) < k.pTol) break;
-        beta = tB[1] / rz;
-        rz = tB[1];
-    }
-    for (int t = tid; t < n; t += nth) {
-        const int i = 1 + t / w, j = 1 + t % w;
-        const size_t c = at(d, i, j);
-        pStar[c] = (double)B.x[c];
-        if (j == w) pStar[c + 1] = 0.0;  // p'(:, N-1) = 0 (pressure_solver.cpp:814)
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) st->itersP = it;
-}
-
 // ------------------------------------------------------------------ correction
 // p += pAlpha p' on [1,M-1] x [1,N-1]; u = clamp(u* + clamp(dE (p'_ij - p'_i,j+1)))
 // on U unknowns and the same for v (iterations.cpp:558-597).

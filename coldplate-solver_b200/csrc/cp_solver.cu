@@ -23,6 +23,7 @@
 #include "cp_kernels.cuh"
 #include "cp_mg.cuh"
 #include "cp_sa.cuh"
+#include "cp_pcg.cuh"
 #include "cp_adjoint.cuh"
 #include "cp_batch.cuh"
 
@@ -326,21 +327,6 @@ struct EvRec {
 #define REC_BEGIN(r, k) do { if (r) (r)->begin(c->stream, (k)); } while (0)
 #define REC_END(r) do { if (r) (r)->end(c->stream); } while (0)
 
-template <typename Kern, typename... Args>
-cudaError_t launch_coop(Kern kern, int grid, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 template <typename TC>
 MomSys<TC> mom_sys(cp_ctx* c, int comp) {
     MomSys<TC> s;
@@ -630,7 +616,7 @@ cp_status enqueue_pressure(cp_ctx* c, EvRec* rec = nullptr) {
         CK(launch_coop_cfg(k_pcg_mg<TV>, c->gMg, kMgThreads, kMgDynSmem, c->stream, c->k, c->st,
                            (const double*)c->dE, (const double*)c->dN, B, H, c->pStar, c->partP, c->barP, c->mgMaps));
     } else {
-        CK(launch_coop(k_pcg<TV>, c->gPcg, c->stream, c->k, c->st, (const double*)c->dE, (const double*)c->dN, B,
+        CK(launch_coop_cfg(k_pcg<TV>, c->gPcg, kPcgThreads, 0, c->stream, c->k, c->st, (const double*)c->dE, (const double*)c->dN, B,
                        c->pStar, c->partP, c->barP));
     }
     REC_END(rec);
@@ -915,15 +901,15 @@ cp_status cp_create(const cp_params* prm, cp_ctx** out) {
     if (c->prm.precision == CP_PREC_MIXED) {
         if (c->jacSeq) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<float, true, true>, kJacSegThreads, 0);
         else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<float, true, false>, kJacThreads, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbP, k_pcg<float>, kThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbP, k_pcg<float>, kPcgThreads, 0);
     } else {
         if (c->jacSeq) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<double, false, true>, kJacSegThreads, 0);
         else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<double, false, false>, kJacThreads, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbP, k_pcg<double>, kThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbP, k_pcg<double>, kPcgThreads, 0);
     }
     if (nbJ < 1 || nbP < 1) return bail(fail(CP_ERR_CUDA, "cooperative kernels do not fit on an SM"));
     c->gJac = c->numSMs * (c->jacSeq ? std::min(nbJ, 3) : 1);
-    c->gPcg = c->numSMs * std::min(nbP, 4);
+    c->gPcg = c->numSMs;
     c->gElem = c->numSMs * 4;
     c->nbMass = c->numSMs * 4;
     if (c->gJac > kMaxBlocks || c->gPcg > kMaxBlocks || c->nbMass > kMaxBlocks)
@@ -1262,7 +1248,7 @@ cp_status adjoint_pcg(cp_ctx* c, const KParams& k, const double* dE, const doubl
         CK(launch_coop_cfg(k_pcg_mg<TV>, c->gMg, kMgThreads, kMgDynSmem, c->stream, k, c->adjSt, dE, dN, B, H, out,
                            c->adjPart, c->adjBar, c->mgMaps));
     } else {
-        CK(launch_coop(k_pcg<TV>, c->gPcg, c->stream, k, c->adjSt, dE, dN, B, out, c->adjPart, c->adjBar));
+        CK(launch_coop_cfg(k_pcg<TV>, c->gPcg, kPcgThreads, 0, c->stream, k, c->adjSt, dE, dN, B, out, c->adjPart, c->adjBar));
     }
     return CP_OK;
 }
@@ -1795,9 +1781,9 @@ extern "C" cp_status cp_pressure_noalloc(const cp_params* p, const double* dE, c
     int dev = 0, sms = 0, nbP = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbP, k_pcg<double>, kThreads, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbP, k_pcg<double>, kPcgThreads, 0));
     if (nbP < 1) return fail(CP_ERR_CUDA, "PCG kernel does not fit on an SM");
-    const int gPcg = sms * std::min(nbP, 4), nbMass = sms * 4;
+    const int gPcg = sms, nbMass = sms * 4;
     if (gPcg > kMaxBlocks || nbMass > kMaxBlocks) return fail(CP_ERR_CUDA, "too many SMs");
     // carve the array: status, barrier counter, partial sums, nine working arrays
     Status* dst = reinterpret_cast<Status*>(base);
@@ -1823,7 +1809,7 @@ extern "C" cp_status cp_pressure_noalloc(const cp_params* p, const double* dE, c
     // the RMS columns of k_mass are not reported here; u*/v* stand in for u/v
     k_mass<double><<<nbMass, kThreads, 0, s>>>(k, dst, uStar, vStar, uStar, vStar, B.rhs, partM);
     CK(cudaGetLastError());
-    CK(launch_coop(k_pcg<double>, gPcg, s, k, dst, dE, dN, B, pStar, partP, bar));
+    CK(launch_coop_cfg(k_pcg<double>, gPcg, kPcgThreads, 0, s, k, dst, dE, dN, B, pStar, partP, bar));
     k_noalloc_massmax<<<1, 256, 0, s>>>(partM, nbMass, dst);
     CK(cudaGetLastError());
     Status hs;
