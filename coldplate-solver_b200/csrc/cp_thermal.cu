@@ -12,23 +12,22 @@
 //                   column; P piecewise constant, so every level keeps the
 //                   7-point form and the levels of A^T are the transposes;
 //   k_th_lu         Thomas factors of every column's tridiagonal z-block, per
-//                   level (z is the direction a column thread owns);
+//                   level;
+//   k_th_matrix     the V-cycle from the first level with at most kThApply
+//                   cells down, as a matrix: one column a CTA, the unit vector
+//                   cycled in shared memory;
 //   k_th_bicgstab   persistent cooperative BiCGStab right-preconditioned by
 //                   one V-cycle: damped z-line Jacobi smoothing (one sweep
-//                   down, one up; exact on the one-column level), residual
-//                   restriction fused with the 2 x 2 sums, the prolongation
-//                   formed on the fly in the two post-smoothing passes (the
-//                   residual over cells, then the z-solve over columns,
-//                   staged through shared memory); levels of at most
-//                   kThCtaCols columns run in block 0 alone.  Bounded grid
-//                   barriers, deterministic block sums, AMGCL's stop test
+//                   down, one up), each direction of a level one pass over
+//                   tiles of whole columns (residual or restriction a thread a
+//                   cell, the z-solve from shared memory), the small levels one
+//                   matrix product.  Bounded grid barriers with the dot
+//                   products on them, deterministic sums, AMGCL's stop test
 //                   ||r|| <= rtol ||b||.  The same kernel solves A^T x = rhs
 //                   for the p-norm adjoint;
 //   k_th_sens       dJ/dgamma from the adjoint field, one thread per column.
 // Layout: every array is indexed k Nx Ny + j Nx + i (i contiguous), so the
-// stencil loads of a warp are coalesced and a column thread walks k with
-// stride Nx Ny.
-#include <cuda_pipeline.h>
+// stencil loads of a warp are coalesced.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -64,17 +63,16 @@ cp_status tfail(cp_status s, const char* fmt, ...) {
                          __FILE__, __LINE__);                                                      \
     } while (0)
 
-constexpr int kThThreads = 256;
-constexpr int kThZ = 16;                  // most layers (a column's sweep is kept in shared memory)
-constexpr int kThMaxNz = kThZ;
-#ifndef CP_TH_STAGE
-#define CP_TH_STAGE 6
-#endif
-constexpr int kThStage = CP_TH_STAGE;     // layers per asynchronous staging chunk
-constexpr int kThStageArr = 5;            // arrays staged per layer at most
-constexpr size_t kThSmemBytes = (size_t)(kThZ + kThStageArr * kThStage) * kThThreads * sizeof(double);
+constexpr int kThThreads = 256;           // element-wise kernels
+constexpr int kThMaxNz = 16;              // most layers (a tile holds whole columns: at least 16 of them)
 constexpr int kThMaxLevels = 16;          // 2 x 2 aggregation from up to 2^15 columns per side
-constexpr long long kThCtaCols = 64;      // levels of at most this many columns: block 0 alone
+constexpr long long kThLarge = 1 << 20;   // cells from which the solver runs 1024 threads an SM instead of 512
+constexpr long long kThApply = 1024;      // levels of at most this many cells: their V-cycle is a matrix
+constexpr int kThMatThreads = 128;
+// three vectors of every level from kThApply cells down: halving in one
+// direction only (a level one column wide) they sum to less than twice the
+// first, plus up to one layer stack a level
+constexpr size_t kThMatSmemMax = 3 * sizeof(double) * (size_t)(2 * kThApply + kThMaxLevels * kThMaxNz);
 constexpr double kThOmega = 0.8;          // z-line Jacobi damping
 constexpr double kThScale0 = 1.4;         // coarse-correction factor into level 0
 constexpr double kThScale = 1.4;          // ... into the deeper levels (1.2 / 1.1: 95 / more iterations
@@ -248,21 +246,8 @@ struct ThLevelT {
 };
 using ThLevel = ThLevelT<double>;
 
-// Entries of row q of A (Tr = false) or of A^T (Tr = true) towards the
-// west, east, south, north, lower and upper neighbour.  Row q of A^T holds
-// column q of A: its west entry is the east coefficient of the west cell.
-template <bool Tr, typename T>
-__device__ __forceinline__ T th_cW(const ThSysT<T>& S, long long q) { return __ldg(Tr ? S.aE + (q - 1) : S.aW + q); }
-template <bool Tr, typename T>
-__device__ __forceinline__ T th_cE(const ThSysT<T>& S, long long q) { return __ldg(Tr ? S.aW + (q + 1) : S.aE + q); }
-template <bool Tr, typename T>
-__device__ __forceinline__ T th_cS(const ThSysT<T>& S, long long q, int nx) {
-    return __ldg(Tr ? S.aN + (q - nx) : S.aS + q);
-}
-template <bool Tr, typename T>
-__device__ __forceinline__ T th_cN(const ThSysT<T>& S, long long q, int nx) {
-    return __ldg(Tr ? S.aS + (q + nx) : S.aN + q);
-}
+// Entry of row q of A (Tr = false) or of A^T (Tr = true) towards the lower and
+// upper neighbour.  Row q of A^T holds column q of A.
 template <bool Tr, typename T>
 __device__ __forceinline__ T th_sub(const ThSysT<T>& S, long long q, long long L) {
     return __ldg(Tr ? S.aT + (q - L) : S.aB + q);
@@ -272,18 +257,58 @@ __device__ __forceinline__ T th_sup(const ThSysT<T>& S, long long q, long long L
     return __ldg(Tr ? S.aB + (q + L) : S.aT + q);
 }
 
+// Row q of the operator and its neighbours' indices.  A neighbour outside the
+// level is the cell itself with a zero entry, so that no load waits for a
+// branch: with a branch a neighbour, a cell of a small level took seven load
+// latencies one after the other.
+template <typename T>
+struct ThRow {
+    T p, w, e, s, n, b, t;
+    unsigned qw, qe, qs, qn, qb, qt;
+};
+
+template <bool Tr, typename T>
+__device__ __forceinline__ ThRow<T> th_row(const ThLevelT<T>& F, int Nz, unsigned q, int i, int j, int kk) {
+    const unsigned L = (unsigned)F.ncol, nx = (unsigned)F.nx;
+    const bool hw = i > 0, he = i < F.nx - 1, hs = j > 0, hn = j < F.ny - 1, hb = kk > 0, ht = kk < Nz - 1;
+    ThRow<T> r;
+    r.qw = hw ? q - 1 : q;
+    r.qe = he ? q + 1 : q;
+    r.qs = hs ? q - nx : q;
+    r.qn = hn ? q + nx : q;
+    r.qb = hb ? q - L : q;
+    r.qt = ht ? q + L : q;
+    r.p = __ldg(F.S.aP + q);
+    r.w = __ldg(Tr ? F.S.aE + r.qw : F.S.aW + q);
+    r.e = __ldg(Tr ? F.S.aW + r.qe : F.S.aE + q);
+    r.s = __ldg(Tr ? F.S.aN + r.qs : F.S.aS + q);
+    r.n = __ldg(Tr ? F.S.aS + r.qn : F.S.aN + q);
+    r.b = __ldg(Tr ? F.S.aT + r.qb : F.S.aB + q);
+    r.t = __ldg(Tr ? F.S.aB + r.qt : F.S.aT + q);
+    if (Tr) {
+        r.w = hw ? r.w : T(0);
+        r.e = he ? r.e : T(0);
+        r.s = hs ? r.s : T(0);
+        r.n = hn ? r.n : T(0);
+        r.b = hb ? r.b : T(0);
+        r.t = ht ? r.t : T(0);
+    }
+    return r;
+}
+
 // (op x)_q on a level, op = A or A^T, in the level's arithmetic T (x may be
 // stored narrower: the FP64 matvec of a float preconditioner output)
 template <bool Tr, typename T, typename X>
-__device__ __forceinline__ T th_ax(const ThLevelT<T>& F, int Nz, const X* x, long long q, int i, int j, int kk) {
-    const long long L = F.ncol;
-    T s = __ldg(F.S.aP + q) * T(x[q]);
-    if (i > 0) s += th_cW<Tr>(F.S, q) * T(x[q - 1]);
-    if (i < F.nx - 1) s += th_cE<Tr>(F.S, q) * T(x[q + 1]);
-    if (j > 0) s += th_cS<Tr>(F.S, q, F.nx) * T(x[q - F.nx]);
-    if (j < F.ny - 1) s += th_cN<Tr>(F.S, q, F.nx) * T(x[q + F.nx]);
-    if (kk > 0) s += th_sub<Tr>(F.S, q, L) * T(x[q - L]);
-    if (kk < Nz - 1) s += th_sup<Tr>(F.S, q, L) * T(x[q + L]);
+__device__ __forceinline__ T th_ax(const ThLevelT<T>& F, int Nz, const X* x, unsigned q, int i, int j, int kk) {
+    const ThRow<T> r = th_row<Tr>(F, Nz, q, i, j, kk);
+    const T xp = T(x[q]), xw = T(x[r.qw]), xe = T(x[r.qe]), xs = T(x[r.qs]), xn = T(x[r.qn]), xb = T(x[r.qb]), xt = T(x[r.qt]);
+    T s = r.p * xp;
+    s += r.w * xw;
+    s += r.e * xe;
+    s += r.s * xs;
+    s += r.n * xn;
+    s += r.b * xb;
+    s += r.t * xt;
     return s;
 }
 
@@ -344,192 +369,257 @@ __global__ void k_th_lu(int Nz, ThLevel F) {
     }
 }
 
-// Shared memory of the column sweeps (doubles): ys[kThZ][blockDim] holds a
-// column's forward sweep, st[kThStageArr][kThStage][blockDim] the staged
-// inputs of kThStage layers.  Each thread uses only its own slots, so no
-// block barrier is needed around them.
-struct ThSm {
-    double* ys;
-    double* st;
-    // a slot holds one value of type S (double or float) in its first bytes
-    template <typename S = double>
-    __device__ __forceinline__ S& y(int kk) const {
-        return *reinterpret_cast<S*>(ys + kk * blockDim.x + threadIdx.x);
+// A tile: W = blockDim / Nz whole columns of a level (in column order, so a
+// tile may span rows), a thread a cell: layer kk, tile column c.  The z-solve
+// of a tile runs from shared memory, a thread a column: the cell threads store
+// f = r inv and g = sub inv and lc, so that a step of either sweep is one
+// multiply-add, y = f - g y and x = y - lc x.
+template <typename T>
+struct ThTile {
+    T *f, *g, *lc, *x;      // [Nz][W] each
+    int W, kk, c;
+    bool on;                // the thread has a cell (kk < Nz)
+    __device__ __forceinline__ int at() const { return kk * W + c; }
+    // one cell's share of the z-block M x = r
+    __device__ __forceinline__ void put(T r, T inv, T sub, T l) const {
+        f[at()] = r * inv;
+        g[at()] = sub * inv;
+        lc[at()] = l;
     }
-    template <typename S = double>
-    __device__ __forceinline__ S& s(int a, int u) const {
-        return *reinterpret_cast<S*>(st + (a * kThStage + u) * blockDim.x + threadIdx.x);
+    // after it x holds M^-1 r; the caller may put the next tile's cells at
+    // once, since f, g, lc are not read any more and the next solve's first
+    // barrier orders the reads of x
+    __device__ __forceinline__ void solve(int Nz) const {
+        __syncthreads();
+        if (threadIdx.x < W) {
+            const T* __restrict__ F = f + threadIdx.x;
+            const T* __restrict__ G = g + threadIdx.x;
+            const T* __restrict__ C = lc + threadIdx.x;
+            T* __restrict__ X = x + threadIdx.x;
+            T v = T(0);
+#pragma unroll 4
+            for (int k = 0; k < Nz; ++k) {
+                v = F[k * W] - G[k * W] * v;
+                X[k * W] = v;
+            }
+            v = T(0);
+#pragma unroll 4
+            for (int k = Nz - 1; k >= 0; --k) {
+                v = X[k * W] - C[k * W] * v;
+                X[k * W] = v;
+            }
+        }
+        __syncthreads();
     }
 };
 
-template <typename S>
-__device__ __forceinline__ void th_stage(S* dst, const S* src) { __pipeline_memcpy_async(dst, src, sizeof(S)); }
-
-// Pre-smoothing from zero over the columns of a level: b = A0 + c1 A1 +
-// c2 A2 (A1, A2 optional; stored to bout when set), x = omega Mz^-1 b.  The
-// inputs of kThStage layers are copied to shared memory asynchronously, all
-// in flight together, and the Thomas recurrence runs from shared memory.
-// T is the level's type, B the type of the right-hand side's terms (double
-// at level 0, where b is a Krylov vector; T on the coarse levels).
-template <bool Tr, typename T, typename B>
-__device__ __forceinline__ void th_presmooth(const ThLevelT<T>& F, int Nz, const B* A0, const B* A1, double c1,
-                                             const B* A2, double c2, B* bout, T* x, double omega, long long t0,
-                                             long long nt, const ThSm& sm) {
-    const long long L = F.ncol;
-    for (long long col = t0; col < F.ncol; col += nt) {
-        T yprev = T(0);
-        for (int k0 = 0; k0 < Nz; k0 += kThStage) {
-            const int nu = min(kThStage, Nz - k0);
-            for (int u = 0; u < nu; ++u) {
-                const int kk = k0 + u;
-                const long long q = kk * L + col;
-                th_stage(&sm.s<B>(0, u), A0 + q);
-                if (A1) th_stage(&sm.s<B>(1, u), A1 + q);
-                if (A2) th_stage(&sm.s<B>(2, u), A2 + q);
-                if (kk > 0) th_stage(&sm.s<T>(3, u), Tr ? F.S.aT + (q - L) : F.S.aB + q);
-                th_stage(&sm.s<T>(4, u), F.linv + q);
-            }
-            __pipeline_commit();
-            __pipeline_wait_prior(0);
-            for (int u = 0; u < nu; ++u) {
-                const int kk = k0 + u;
-                B b = sm.s<B>(0, u);
-                if (A1) b += c1 * sm.s<B>(1, u);
-                if (A2) b += c2 * sm.s<B>(2, u);
-                if (bout) bout[kk * L + col] = b;
-                const T sub = kk > 0 ? sm.s<T>(3, u) : T(0);
-                yprev = (T(b) - sub * yprev) * sm.s<T>(4, u);
-                sm.y<T>(kk) = yprev;
-            }
-        }
-        T xn = T(0);
-        for (int k0 = ((Nz - 1) / kThStage) * kThStage; k0 >= 0; k0 -= kThStage) {
-            const int nu = min(kThStage, Nz - k0);
-            for (int u = 0; u < nu; ++u) {
-                const int kk = k0 + u;
-                if (kk < Nz - 1) th_stage(&sm.s<T>(0, u), F.lc + (kk * L + col));
-            }
-            __pipeline_commit();
-            __pipeline_wait_prior(0);
-            for (int u = nu - 1; u >= 0; --u) {
-                const int kk = k0 + u;
-                const T xv = sm.y<T>(kk) - (kk < Nz - 1 ? sm.s<T>(0, u) * xn : T(0));
-                x[kk * L + col] = T(omega) * xv;
-                xn = xv;
-            }
-        }
-    }
-}
-
-// Residual restriction: bC = sum over the 2 x 2 aggregate of (bF - op xF).
-// The four fine residuals are independent, so their loads are in flight
-// together; index math in 32 bits (levels hold fewer than 2^31 cells).
-template <bool Tr, typename T, typename B>
-__device__ __forceinline__ void th_restrict(const ThLevelT<T>& F, const ThLevelT<T>& C, int Nz, const B* bF,
-                                            const T* xF, T* bC, long long t0, long long nt) {
-    const unsigned LC = (unsigned)C.ncol, cnx = (unsigned)C.nx, LF = (unsigned)F.ncol;
-    for (unsigned qc = (unsigned)t0; qc < (unsigned)C.n; qc += (unsigned)nt) {
-        const unsigned kk = qc / LC, rem = qc - kk * LC, J = rem / cnx, I = rem - J * cnx;
-        T r[4];
-#pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            const int i = 2 * (int)I + (d & 1), j = 2 * (int)J + (d >> 1);
-            r[d] = T(0);
-            if (i < F.nx && j < F.ny) {
-                const long long q = (long long)kk * LF + (long long)j * F.nx + i;
-                r[d] = T(bF[q]) - th_ax<Tr>(F, Nz, xF, q, i, j, (int)kk);
-            }
-        }
-        bC[qc] = ((r[0] + r[1]) + r[2]) + r[3];
-    }
-}
-
-// Post-smoothing, first half (cells): out = bF - op xp with the prolonged
-// iterate xp = xF + scale P xC formed on the fly at every stencil point.
-// Two cells a thread per step (their loads in flight together), 32-bit
-// index math.
-template <bool Tr, typename T, typename B>
-__device__ __forceinline__ T th_post_res1(const ThLevelT<T>& F, const ThLevelT<T>& C, int Nz, const B* bF,
-                                          const T* xF, const T* xC, T scale, unsigned q) {
-    const unsigned L = (unsigned)F.ncol, LC = (unsigned)C.ncol, nx = (unsigned)F.nx, cnx = (unsigned)C.nx;
-    const unsigned kk = q / L, col = q - kk * L, ju = col / nx, iu = col - ju * nx;
-    const int i = (int)iu, j = (int)ju;
-    const unsigned kc = kk * LC, cj = (ju >> 1) * cnx;
-    T ax = __ldg(F.S.aP + q) * (xF[q] + scale * xC[kc + cj + (iu >> 1)]);
-    if (i > 0) ax += th_cW<Tr>(F.S, q) * (xF[q - 1] + scale * xC[kc + cj + ((iu - 1) >> 1)]);
-    if (i < F.nx - 1) ax += th_cE<Tr>(F.S, q) * (xF[q + 1] + scale * xC[kc + cj + ((iu + 1) >> 1)]);
-    if (j > 0) ax += th_cS<Tr>(F.S, q, F.nx) * (xF[q - nx] + scale * xC[kc + ((ju - 1) >> 1) * cnx + (iu >> 1)]);
-    if (j < F.ny - 1)
-        ax += th_cN<Tr>(F.S, q, F.nx) * (xF[q + nx] + scale * xC[kc + ((ju + 1) >> 1) * cnx + (iu >> 1)]);
-    if (kk > 0) ax += th_sub<Tr>(F.S, q, L) * (xF[q - L] + scale * xC[kc - LC + cj + (iu >> 1)]);
-    if ((int)kk < Nz - 1) ax += th_sup<Tr>(F.S, q, L) * (xF[q + L] + scale * xC[kc + LC + cj + (iu >> 1)]);
-    return T(bF[q]) - ax;
-}
-
-template <bool Tr, typename T, typename B>
-__device__ __forceinline__ void th_post_resid(const ThLevelT<T>& F, const ThLevelT<T>& C, int Nz, const B* bF,
-                                              const T* xF, const T* xC, double scale, T* out, long long t0,
-                                              long long nt) {
-    const unsigned n = (unsigned)F.n, st = (unsigned)nt;
-    const T sc = T(scale);
-    unsigned q = (unsigned)t0;
-    for (; q + st < n; q += 2 * st) {
-        const T r0 = th_post_res1<Tr>(F, C, Nz, bF, xF, xC, sc, q);
-        const T r1 = th_post_res1<Tr>(F, C, Nz, bF, xF, xC, sc, q + st);
-        out[q] = r0;
-        out[q + st] = r1;
-    }
-    if (q < n) out[q] = th_post_res1<Tr>(F, C, Nz, bF, xF, xC, sc, q);
-}
-
-// Post-smoothing, second half (columns): out = xp + omega Mz^-1 out, in
-// place (each column reads its residual before writing the result)
+// Entry below of the z-block and the Thomas factors of a cell
 template <bool Tr, typename T>
-__device__ __forceinline__ void th_post_cols(const ThLevelT<T>& F, const ThLevelT<T>& C, int Nz, const T* xF,
-                                             const T* xC, double scale, double omega, T* out, long long t0,
-                                             long long nt, const ThSm& sm) {
-    const long long L = F.ncol, LC = C.ncol;
-    for (long long col = t0; col < F.ncol; col += nt) {
-        const int i = (int)(col % F.nx), j = (int)(col / F.nx);
-        const long long c0 = (long long)(j >> 1) * C.nx + (i >> 1);
-        T yprev = T(0);
-        for (int k0 = 0; k0 < Nz; k0 += kThStage) {
-            const int nu = min(kThStage, Nz - k0);
-            for (int u = 0; u < nu; ++u) {
-                const int kk = k0 + u;
-                const long long q = kk * L + col;
-                th_stage(&sm.s<T>(0, u), out + q);
-                if (kk > 0) th_stage(&sm.s<T>(1, u), Tr ? F.S.aT + (q - L) : F.S.aB + q);
-                th_stage(&sm.s<T>(2, u), F.linv + q);
-            }
-            __pipeline_commit();
-            __pipeline_wait_prior(0);
-            for (int u = 0; u < nu; ++u) {
-                const int kk = k0 + u;
-                const T sub = kk > 0 ? sm.s<T>(1, u) : T(0);
-                yprev = (sm.s<T>(0, u) - sub * yprev) * sm.s<T>(2, u);
-                sm.y<T>(kk) = yprev;
-            }
+__device__ __forceinline__ void th_zrow(const ThLevelT<T>& F, unsigned q, int kk, T& inv, T& sub, T& l) {
+    const unsigned L = (unsigned)F.ncol, qb = kk > 0 ? q - L : q;
+    inv = __ldg(F.linv + q);
+    l = __ldg(F.lc + q);
+    sub = __ldg(Tr ? F.S.aT + qb : F.S.aB + q);
+    if (kk == 0) sub = T(0);
+}
+
+// Pre-smoothing from zero on level 0, with the vector update that makes its
+// right-hand side: b = A0 + c1 A1 + c2 A2 (A2 optional; stored to bout),
+// x = omega Mz^-1 b.
+template <bool Tr, typename T>
+__device__ __forceinline__ void th_presmooth(const ThLevelT<T>& F, int Nz, const double* A0, const double* A1, double c1,
+                                             const double* A2, double c2, double* bout, double omega, const ThTile<T>& t) {
+    const unsigned L = (unsigned)F.ncol;
+    for (unsigned c0 = blockIdx.x * t.W; c0 < L; c0 += gridDim.x * t.W) {
+        const unsigned col = c0 + t.c, q = t.kk * L + col;
+        const bool on = t.on && col < L;
+        if (on) {
+            T inv, sub, l;
+            th_zrow<Tr>(F, q, t.kk, inv, sub, l);
+            double b = A0[q];
+            const double a1 = A1[q], a2 = A2 ? A2[q] : 0.0;
+            b += c1 * a1;
+            if (A2) b += c2 * a2;
+            bout[q] = b;
+            t.put(T(b), inv, sub, l);
         }
-        T cnext = T(0);
-        for (int k0 = ((Nz - 1) / kThStage) * kThStage; k0 >= 0; k0 -= kThStage) {
-            const int nu = min(kThStage, Nz - k0);
-            for (int u = 0; u < nu; ++u) {
-                const int kk = k0 + u;
-                const long long q = kk * L + col;
-                if (kk < Nz - 1) th_stage(&sm.s<T>(0, u), F.lc + q);
-                th_stage(&sm.s<T>(1, u), xF + q);
-                th_stage(&sm.s<T>(2, u), xC + (kk * LC + c0));
+        t.solve(Nz);
+        if (on) F.x[q] = T(omega) * t.x[t.at()];
+    }
+}
+
+// Descent from level F to C: b_C = the sum over the 2 x 2 aggregate of
+// b - op x, and the pre-smoothing of C, x_C = omega Mz^-1 b_C (unless C is
+// solved by its matrix, `last`).  A thread a coarse cell, its four fine
+// residuals' loads in flight two by two.
+template <bool Tr, typename T, typename B>
+__device__ __forceinline__ void th_down(const ThLevelT<T>& F, const ThLevelT<T>& C, int Nz, const B* bF, double omega,
+                                        bool last, const ThTile<T>& t) {
+    const unsigned LF = (unsigned)F.ncol, LC = (unsigned)C.ncol, cnx = (unsigned)C.nx;
+    for (unsigned c0 = blockIdx.x * t.W; c0 < LC; c0 += gridDim.x * t.W) {
+        const unsigned col = c0 + t.c, qc = t.kk * LC + col;
+        const bool on = t.on && col < LC;
+        if (on) {
+            const unsigned J = col / cnx, I = col - J * cnx;
+            T inv = T(0), sub = T(0), l = T(0);
+            if (!last) th_zrow<Tr>(C, qc, t.kk, inv, sub, l);
+            T b = T(0);
+#pragma unroll 1
+            for (int d = 0; d < 4; ++d) {
+                const int i = 2 * (int)I + (d & 1), j = 2 * (int)J + (d >> 1);
+                // an odd edge's missing cell is read inside and dropped
+                const int ii = min(i, F.nx - 1), jj = min(j, F.ny - 1);
+                const unsigned q = t.kk * LF + (unsigned)jj * F.nx + ii;
+                const T v = T(bF[q]) - th_ax<Tr>(F, Nz, F.x, q, ii, jj, t.kk);
+                b += (i < F.nx && j < F.ny) ? v : T(0);
             }
-            __pipeline_commit();
-            __pipeline_wait_prior(0);
-            for (int u = nu - 1; u >= 0; --u) {
-                const int kk = k0 + u;
-                const T corr = sm.y<T>(kk) - (kk < Nz - 1 ? sm.s<T>(0, u) * cnext : T(0));
-                out[kk * L + col] = sm.s<T>(1, u) + T(scale) * sm.s<T>(2, u) + T(omega) * corr;
-                cnext = corr;
-            }
+            C.b[qc] = b;
+            if (!last) t.put(b, inv, sub, l);
         }
+        if (last) continue;
+        t.solve(Nz);
+        if (on) C.x[qc] = T(omega) * t.x[t.at()];
+    }
+}
+
+// Ascent from level C to F with the post-smoothing: xp = x + scale P xC formed
+// at every stencil point, out = xp + omega Mz^-1 (b - op xp).
+template <bool Tr, typename T, typename B>
+__device__ __forceinline__ void th_up(const ThLevelT<T>& F, const ThLevelT<T>& C, int Nz, const B* bF, const T* xC,
+                                      double scale, double omega, T* out, const ThTile<T>& t) {
+    const unsigned L = (unsigned)F.ncol, LC = (unsigned)C.ncol, nx = (unsigned)F.nx, cnx = (unsigned)C.nx;
+    const T sc = T(scale);
+    const T* xF = F.x;
+    for (unsigned c0 = blockIdx.x * t.W; c0 < L; c0 += gridDim.x * t.W) {
+        const unsigned col = c0 + t.c, q = t.kk * L + col;
+        const bool on = t.on && col < L;
+        T xp = T(0);
+        if (on) {
+            const unsigned ju = col / nx, iu = col - ju * nx;
+            const int i = (int)iu, j = (int)ju;
+            const ThRow<T> r = th_row<Tr>(F, Nz, q, i, j, t.kk);
+            T inv, sub, l;
+            th_zrow<Tr>(F, q, t.kk, inv, sub, l);
+            // the parents: a neighbour's is the cell's own or the one across
+            const unsigned kc = t.kk * LC, I = iu >> 1, J = ju >> 1;
+            const unsigned Iw = i > 0 ? (iu - 1) >> 1 : I, Ie = i < F.nx - 1 ? (iu + 1) >> 1 : I;
+            const unsigned Js = j > 0 ? (ju - 1) >> 1 : J, Jn = j < F.ny - 1 ? (ju + 1) >> 1 : J;
+            const unsigned kb = t.kk > 0 ? kc - LC : kc, kt = t.kk < Nz - 1 ? kc + LC : kc;
+            const T cp = xC[kc + J * cnx + I], cw = xC[kc + J * cnx + Iw], ce = xC[kc + J * cnx + Ie],
+                    cs = xC[kc + Js * cnx + I], cn = xC[kc + Jn * cnx + I], cb = xC[kb + J * cnx + I],
+                    ct = xC[kt + J * cnx + I];
+            const T fp = xF[q], fw = xF[r.qw], fe = xF[r.qe], fs = xF[r.qs], fn = xF[r.qn], fb = xF[r.qb], ft = xF[r.qt];
+            const T bq = T(bF[q]);
+            xp = fp + sc * cp;
+            T ax = r.p * xp;
+            ax += r.w * (fw + sc * cw);
+            ax += r.e * (fe + sc * ce);
+            ax += r.s * (fs + sc * cs);
+            ax += r.n * (fn + sc * cn);
+            ax += r.b * (fb + sc * cb);
+            ax += r.t * (ft + sc * ct);
+            t.put(bq - ax, inv, sub, l);
+        }
+        t.solve(Nz);
+        if (on) out[q] = xp + T(omega) * t.x[t.at()];
+    }
+}
+
+// y = B b on the level that is solved by its matrix, a warp a row
+template <typename T>
+__device__ __forceinline__ void th_apply(const ThLevelT<T>& F, const T* __restrict__ bm) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = gridDim.x * (blockDim.x >> 5), n = (int)F.n;
+    for (int i = wid * gridDim.x + blockIdx.x; i < n; i += nw) {
+        const T* row = bm + (size_t)i * n;
+        T s = T(0);
+#pragma unroll 16
+        for (int q = lane; q < n; q += 32) s += row[q] * F.b[q];
+        s = warp_sum(s);
+        if (lane == 0) F.y[i] = s;
+    }
+}
+
+// out = w Mz^-1 r of a level's columns, from and to shared memory (in place
+// allowed), a thread a column
+template <bool Tr>
+__device__ __forceinline__ void th_mat_zsolve(const ThLevel& F, int Nz, const double* r, double w, double* out) {
+    const int L = (int)F.ncol;
+    for (int c = threadIdx.x; c < L; c += blockDim.x) {
+        double y = 0.0;
+        for (int k = 0; k < Nz; ++k) {
+            const int q = k * L + c;
+            y = (r[q] - (k > 0 ? th_sub<Tr>(F.S, q, L) : 0.0) * y) * F.linv[q];
+            out[q] = y;
+        }
+        double x = 0.0;
+        for (int k = Nz - 1; k >= 0; --k) {
+            const int q = k * L + c;
+            x = out[q] - (k < Nz - 1 ? F.lc[q] * x : 0.0);
+            out[q] = w * x;
+        }
+    }
+    __syncthreads();
+}
+
+// Column q of the V-cycle's matrix on levels [m, L): the cycle of the unit
+// vector e_q in shared memory (b, x, y of every level), a CTA a column.
+template <bool Tr, typename T>
+__global__ void __launch_bounds__(kThMatThreads) k_th_matrix(int Nz, const ThLevel* __restrict__ lv, int m, int L,
+                                                             double omega, double scale, T* bm) {
+    extern __shared__ double sh[];
+    __shared__ double* at[kThMaxLevels];
+    const int n = (int)lv[m].n;
+    if (threadIdx.x == 0) {
+        double* p = sh;
+        for (int l = m; l < L; ++l) {
+            at[l] = p;
+            p += 3 * lv[l].n;
+        }
+    }
+    __syncthreads();
+    for (int q0 = blockIdx.x; q0 < n; q0 += gridDim.x) {
+        for (int q = threadIdx.x; q < n; q += blockDim.x) at[m][q] = q == q0 ? 1.0 : 0.0;
+        __syncthreads();
+        for (int l = m;; ++l) {
+            const ThLevel F = lv[l];
+            double *b = at[l], *x = b + F.n;
+            th_mat_zsolve<Tr>(F, Nz, b, l + 1 == L ? 1.0 : omega, x);
+            if (l + 1 == L) break;
+            const ThLevel C = lv[l + 1];
+            for (int qc = threadIdx.x; qc < (int)C.n; qc += blockDim.x) {
+                const int kk = qc / (int)C.ncol, rem = qc - kk * (int)C.ncol, J = rem / C.nx, I = rem - J * C.nx;
+                double r = 0.0;
+                for (int d = 0; d < 4; ++d) {
+                    const int i = 2 * I + (d & 1), j = 2 * J + (d >> 1);
+                    if (i >= F.nx || j >= F.ny) continue;
+                    const unsigned q = (unsigned)(kk * (int)F.ncol + j * F.nx + i);
+                    r += b[q] - th_ax<Tr>(F, Nz, x, q, i, j, kk);
+                }
+                at[l + 1][qc] = r;
+            }
+            __syncthreads();
+        }
+        for (int l = L - 2; l >= m; --l) {
+            const ThLevel F = lv[l], C = lv[l + 1];
+            double *b = at[l], *x = b + F.n, *y = x + F.n;
+            const double* xc = at[l + 1] + (l + 2 == L ? 1 : 2) * C.n;
+            for (int q = threadIdx.x; q < (int)F.n; q += blockDim.x) {
+                const int kk = q / (int)F.ncol, rem = q - kk * (int)F.ncol, j = rem / F.nx, i = rem - j * F.nx;
+                x[q] += scale * xc[kk * (int)C.ncol + (j >> 1) * C.nx + (i >> 1)];
+            }
+            __syncthreads();
+            for (int q = threadIdx.x; q < (int)F.n; q += blockDim.x) {
+                const int kk = q / (int)F.ncol, rem = q - kk * (int)F.ncol, j = rem / F.nx, i = rem - j * F.nx;
+                y[q] = b[q] - th_ax<Tr>(F, Nz, x, (unsigned)q, i, j, kk);
+            }
+            __syncthreads();
+            th_mat_zsolve<Tr>(F, Nz, y, omega, y);
+            for (int q = threadIdx.x; q < (int)F.n; q += blockDim.x) y[q] += x[q];
+            __syncthreads();
+        }
+        const double* out = at[m] + (m + 1 == L ? 1 : 2) * n;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) bm[(size_t)i * n + q0] = (T)out[i];
+        __syncthreads();
     }
 }
 
@@ -537,19 +627,19 @@ __device__ __forceinline__ void th_post_cols(const ThLevelT<T>& F, const ThLevel
 // assembled system when T is float)
 template <typename T>
 struct ThHierT {
-    int L, cta;             // levels; first level run by block 0 alone (L: none)
+    int L, m;               // levels; the V-cycle from level m (>= 1) down is the matrix bm
     double omega, scale0, scale;   // coarse-correction factor into level 0, into the deeper levels
     const ThLevelT<T>* lv;  // device array of L levels
+    T* bm;                  // n x n for the n cells of level m
     unsigned long long* prof;  // per-phase nanoseconds (CP_TH_PROFILE), or null
 };
 using ThHier = ThHierT<double>;
 
 // phase slots of the profile: the BiCGStab phases, then 16 slots per
-// V-cycle phase kind indexed by level
+// V-cycle direction indexed by level
 enum ThProfSlot {
     TH_P_INIT = 0, TH_P_PRE_P = 1, TH_P_MATVEC_V = 2, TH_P_PRE_S = 3, TH_P_MATVEC_T = 4, TH_P_UPDATE = 5,
-    TH_P_BLOCK0 = 6, TH_P_RESTRICT = 16, TH_P_PRESMOOTH = 32, TH_P_POSTRES = 48, TH_P_POSTCOL = 64,
-    TH_P_COUNT = 80
+    TH_P_APPLY = 6, TH_P_DOWN = 16, TH_P_UP = 32, TH_P_COUNT = 48
 };
 
 // BiCGStab's vectors, FP64; the preconditioned directions ph = M^-1 p and
@@ -565,216 +655,165 @@ using ThVecs = ThVecsT<double>;
 // A x = rhs (Tr = false) or A^T x = rhs (Tr = true), from the x in V.x.
 // F0 is the FP64 system (matvecs, residuals, dot products); the V-cycle runs
 // on H in type T (T = float: the mixed-precision form; T = double: H.lv[0]
-// is F0).  Dynamic shared memory: kThSmemBytes (the column sweeps' staging).
-template <bool Tr, typename T>
-__global__ void __launch_bounds__(kThThreads, 2) k_th_bicgstab(ThK k, ThLevel F0, ThHierT<T> H, const double* rhs,
+// is F0).
+// Two V-cycles, two matvecs and an update an iteration: 2 (2 m + 3) + 3
+// barriers, 27 at 151 x 97 x 9 and 37 at 1024 x 512 x 12.  At the small end
+// these are the cost; an iteration takes 94 us there instead of 310.  At
+// 1024 x 512 x 12 the passes over level 0 are, bound by their loads (the seven
+// coefficient arrays first): 1.20 ms instead of 1.85.
+// NT threads a CTA, two CTAs an SM: 256 (128 registers, no spills) where the
+// barriers are the cost, 512 from kThLarge
+// cells on, where more warps in flight are worth more (1.20 against 1.46 ms an
+// iteration at 1024 x 512 x 12; 94 against 113 us at 151 x 97 x 9).
+template <bool Tr, typename T, int NT>
+__global__ void __launch_bounds__(NT, 2) k_th_bicgstab(ThK k, ThLevel F0, ThHierT<T> H, const double* rhs,
                                                               ThVecsT<T> V, double* part, unsigned* bar, ThStatus* st,
                                                               int maxiter, double rtol) {
-    __shared__ double sm[96];
-    extern __shared__ double th_dyn[];
-    const ThSm cs{th_dyn, th_dyn + kThZ * blockDim.x};
-    const int G = gridDim.x, Nz = k.Nz;
-    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nth = (long long)G * blockDim.x;
+    __shared__ double sm[kReduceSm];
+    __shared__ ThLevelT<T> lv[kThMaxLevels];
+    __shared__ T tile[4][NT];
+    const int Nz = k.Nz;
+    const unsigned tid = blockIdx.x * NT + threadIdx.x, nth = gridDim.x * NT;
+    const Team team = grid_team(bar, &st->err);
     unsigned target = 0;
-    double* pA = part;             // [G][2]
-    double* pB = part + 2 * G;     // [G][2]
-    double* pC = part + 4 * G;     // [G][2]
-    unsigned long long tprev = (H.prof && blockIdx.x == 0 && threadIdx.x == 0) ? globaltimer_ns() : 0ull;
-    // grid barrier; with the profile on, block 0 books the time since the
-    // previous barrier to the phase slot
-    auto sync = [&](int slot) -> bool {
-        target += G;
-        const bool ok = grid_barrier(bar, target, &st->err);
-        if (H.prof && blockIdx.x == 0 && threadIdx.x == 0) {
+    for (int l = threadIdx.x; l < H.L; l += NT) lv[l] = H.lv[l];
+    ThTile<T> tl;
+    tl.f = tile[0]; tl.g = tile[1]; tl.lc = tile[2]; tl.x = tile[3];
+    tl.W = NT / Nz;
+    tl.kk = threadIdx.x / tl.W;
+    tl.c = threadIdx.x - tl.kk * tl.W;
+    tl.on = tl.kk < Nz;
+    __syncthreads();
+    unsigned long long tprev = (H.prof && team.lead()) ? globaltimer_ns() : 0ull;
+    // with the profile on, block 0 books the time since the previous barrier
+    // to the phase slot
+    auto tick = [&](int slot) {
+        if (H.prof && team.lead()) {
             const unsigned long long t = globaltimer_ns();
             H.prof[slot] += t - tprev;
             tprev = t;
         }
+    };
+    auto sync = [&](int slot) -> bool {
+        const bool ok = team_sync(team, target);
+        tick(slot);
         return ok;
     };
-    auto cells = [&](auto&& fn) {
-        for (long long q = tid; q < k.n; q += nth) {
-            const int kk = (int)(q / k.ncol);
-            const long long rem = q - kk * k.ncol;
-            fn(q, (int)(rem % k.Nx), (int)(rem / k.Nx), kk);
-        }
+    auto reduce = [&](int slot, double (&v)[2]) -> bool {
+        const bool ok = team_reduce(team, target, v, part, sm);
+        tick(slot);
+        return ok;
     };
     // Two cells a thread per step: compute(q, i, j, kk) only loads and
     // computes (its loads for both cells in flight together), commit(q, v)
     // stores and accumulates; 32-bit index math.
     auto cells2 = [&](auto&& compute, auto&& commit) {
-        const unsigned n = (unsigned)k.n, L = (unsigned)k.ncol, nx = (unsigned)k.Nx, stp = (unsigned)nth;
+        const unsigned n = (unsigned)k.n, L = (unsigned)k.ncol, nx = (unsigned)k.Nx;
         auto at = [&](unsigned q) {
             const unsigned kk = q / L, rem = q - kk * L, j = rem / nx;
-            return compute((long long)q, (int)(rem - j * nx), (int)j, (int)kk);
+            return compute(q, (int)(rem - j * nx), (int)j, (int)kk);
         };
-        unsigned q = (unsigned)tid;
-        for (; q + stp < n; q += 2 * stp) {
+        unsigned q = tid;
+        for (; q < n && n - q > nth; q += 2 * nth) {
             const auto a = at(q);
-            const auto b = at(q + stp);
-            commit((long long)q, a);
-            commit((long long)(q + stp), b);
+            const auto b = at(q + nth);
+            commit(q, a);
+            commit(q + nth, b);
         }
-        if (q < n) commit((long long)q, at(q));
+        if (q < n) commit(q, at(q));
     };
-    // The V-cycle after the level-0 pre-smoothing (H.lv[0].x = omega Mz^-1 b0):
+    // The V-cycle after the level-0 pre-smoothing (lv[0].x = omega Mz^-1 b0):
     // out0 = M^-1 b0.  Ends with a grid barrier.
     auto vcycle = [&](const double* b0, T* out0) __attribute__((always_inline)) -> bool {
-        const int L = H.L;
-        // residual restriction from level l (its right-hand side: b0 at level 0)
-        auto restrict_from = [&](int l) __attribute__((always_inline)) {
-            const ThLevelT<T> &F = H.lv[l], &C = H.lv[l + 1];
-            if (l == 0) th_restrict<Tr>(F, C, Nz, b0, F.x, C.b, tid, nth);
-            else th_restrict<Tr>(F, C, Nz, F.b, F.x, C.b, tid, nth);
-        };
-        int l = 0;
-        for (; l + 1 < L && l + 1 < H.cta; ++l) {
-            const ThLevelT<T>& C = H.lv[l + 1];
-            restrict_from(l);
-            if (!sync(TH_P_RESTRICT + l)) return false;
-            th_presmooth<Tr>(C, Nz, C.b, (const T*)nullptr, 0.0, (const T*)nullptr, 0.0, (T*)nullptr, C.x,
-                             l + 2 == L ? 1.0 : H.omega, tid, nth, cs);
-            if (!sync(TH_P_PRESMOOTH + l + 1)) return false;
+        for (int l = 0; l < H.m; ++l) {
+            if (l == 0) th_down<Tr>(lv[0], lv[1], Nz, b0, H.omega, H.m == 1, tl);
+            else th_down<Tr>(lv[l], lv[l + 1], Nz, (const T*)lv[l].b, H.omega, l + 1 == H.m, tl);
+            if (!sync(TH_P_DOWN + l)) return false;
         }
-        if (l + 1 < L) {
-            // levels l+1 .. L-1 are small: restrict to l+1 grid-wide, then block 0
-            restrict_from(l);
-            if (!sync(TH_P_RESTRICT + l)) return false;
-            if (blockIdx.x == 0) {
-                const long long bt = threadIdx.x, bn = blockDim.x;
-                for (int m = l + 1;; ++m) {
-                    const ThLevelT<T>& C = H.lv[m];
-                    th_presmooth<Tr>(C, Nz, C.b, (const T*)nullptr, 0.0, (const T*)nullptr, 0.0, (T*)nullptr, C.x,
-                                     m + 1 == L ? 1.0 : H.omega, bt, bn, cs);
-                    __syncthreads();
-                    if (m + 1 == L) break;
-                    th_restrict<Tr>(C, H.lv[m + 1], Nz, C.b, C.x, H.lv[m + 1].b, bt, bn);
-                    __syncthreads();
-                }
-                for (int m = L - 2; m >= l + 1; --m) {
-                    const ThLevelT<T> &F = H.lv[m], &C = H.lv[m + 1];
-                    const T* xc = m + 2 == L ? C.x : C.y;
-                    th_post_resid<Tr>(F, C, Nz, F.b, F.x, xc, H.scale, F.y, bt, bn);
-                    __syncthreads();
-                    th_post_cols<Tr>(F, C, Nz, F.x, xc, H.scale, H.omega, F.y, bt, bn, cs);   // m >= 1
-                    __syncthreads();
-                }
-            }
-            if (!sync(TH_P_BLOCK0)) return false;
-        } else {
-            l = L - 2;   // every level grid-wide: the ascent starts above the bottom
-        }
-        for (int m = l; m >= 0; --m) {
-            const ThLevelT<T> &F = H.lv[m], &C = H.lv[m + 1];
-            const T* xc = m + 2 == L ? C.x : C.y;
-            T* out = m == 0 ? out0 : F.y;
-            const double sc = m == 0 ? H.scale0 : H.scale;
-            if (m == 0) th_post_resid<Tr>(F, C, Nz, b0, F.x, xc, sc, out, tid, nth);
-            else th_post_resid<Tr>(F, C, Nz, F.b, F.x, xc, sc, out, tid, nth);
-            if (!sync(TH_P_POSTRES + m)) return false;
-            th_post_cols<Tr>(F, C, Nz, F.x, xc, sc, H.omega, out, tid, nth, cs);
-            if (!sync(TH_P_POSTCOL + m)) return false;
+        th_apply(lv[H.m], H.bm);
+        if (!sync(TH_P_APPLY)) return false;
+        for (int l = H.m - 1; l >= 0; --l) {
+            if (l == 0) th_up<Tr>(lv[0], lv[1], Nz, b0, lv[1].y, H.scale0, H.omega, out0, tl);
+            else th_up<Tr>(lv[l], lv[l + 1], Nz, (const T*)lv[l].b, lv[l + 1].y, H.scale, H.omega, lv[l].y, tl);
+            if (!sync(TH_P_UP + l)) return false;
         }
         return true;
     };
     // ---- r = rhs - op x, rh = r, p = v = 0; ||rhs||^2, ||r||^2
-    {
-        double acc[2] = {0.0, 0.0};
-        cells([&](long long q, int i, int j, int kk) {
-            const double r = rhs[q] - th_ax<Tr>(F0, Nz, V.x, q, i, j, kk);
-            V.r[q] = r;
-            V.rh[q] = r;
-            V.p[q] = 0.0;
-            V.v[q] = 0.0;
-            acc[0] += rhs[q] * rhs[q];
-            acc[1] += r * r;
-        });
-        block_sum<2>(acc, sm);
-        if (threadIdx.x == 0) { pC[2 * blockIdx.x] = acc[0]; pC[2 * blockIdx.x + 1] = acc[1]; }
-    }
-    if (!sync(TH_P_INIT)) return;
-    double tot[2];
-    sum_partials<2>(pC, G, 2, tot, sm);
-    const double bnorm = sqrt(tot[0]) > 0.0 ? sqrt(tot[0]) : 1.0;
-    double res = sqrt(tot[1]) / bnorm;
-    double rho = 1.0, alpha = 1.0, omega = 1.0, rho1 = tot[1];
+    double acc[2] = {0.0, 0.0};
+    cells2([&](unsigned q, int i, int j, int kk) {
+        const double b = rhs[q];
+        return make_double2(b, b - th_ax<Tr>(F0, Nz, V.x, q, i, j, kk));
+    }, [&](unsigned q, double2 a) {
+        V.r[q] = a.y;
+        V.rh[q] = a.y;
+        V.p[q] = 0.0;
+        V.v[q] = 0.0;
+        acc[0] += a.x * a.x;
+        acc[1] += a.y * a.y;
+    });
+    if (!reduce(TH_P_INIT, acc)) return;
+    const double bnorm = sqrt(acc[0]) > 0.0 ? sqrt(acc[0]) : 1.0;
+    double res = sqrt(acc[1]) / bnorm;
+    double rho = 1.0, alpha = 1.0, omega = 1.0, rho1 = acc[1];
     int it = 0;
     bool conv = res <= rtol;
     for (; it < maxiter && !conv; ++it) {
         if (rho1 == 0.0) break;
         const double beta = (rho1 / rho) * (alpha / omega);
         // ---- p = r + beta p - beta omega v, fused with the level-0 pre-smoothing; ph = M^-1 p
-        th_presmooth<Tr>(H.lv[0], Nz, (const double*)V.r, (const double*)V.p, beta, (const double*)V.v,
-                         -beta * omega, V.p, H.lv[0].x, H.omega, tid, nth, cs);
+        th_presmooth<Tr>(lv[0], Nz, V.r, V.p, beta, V.v, -beta * omega, V.p, H.omega, tl);
         if (!sync(TH_P_PRE_P)) return;
         if (!vcycle(V.p, V.ph)) return;
         // ---- v = op ph; (rh, v)
-        {
-            double acc[2] = {0.0, 0.0};
-            cells2([&](long long q, int i, int j, int kk) {
-                return make_double2(th_ax<Tr>(F0, Nz, V.ph, q, i, j, kk), V.rh[q]);
-            }, [&](long long q, double2 a) {
-                V.v[q] = a.x;
-                acc[0] += a.y * a.x;
-            });
-            block_sum<2>(acc, sm);
-            if (threadIdx.x == 0) pA[2 * blockIdx.x] = acc[0];
-        }
-        if (!sync(TH_P_MATVEC_V)) return;
-        double rv[2];
-        sum_partials<2>(pA, G, 2, rv, sm);
-        if (rv[0] == 0.0) break;
-        alpha = rho1 / rv[0];
+        acc[0] = acc[1] = 0.0;
+        cells2([&](unsigned q, int i, int j, int kk) {
+            return make_double2(th_ax<Tr>(F0, Nz, V.ph, q, i, j, kk), V.rh[q]);
+        }, [&](unsigned q, double2 a) {
+            V.v[q] = a.x;
+            acc[0] += a.y * a.x;
+        });
+        if (!reduce(TH_P_MATVEC_V, acc)) return;
+        if (acc[0] == 0.0) break;
+        alpha = rho1 / acc[0];
         // ---- s = r - alpha v, fused with the level-0 pre-smoothing; sh = M^-1 s
-        th_presmooth<Tr>(H.lv[0], Nz, (const double*)V.r, (const double*)V.v, -alpha, (const double*)nullptr, 0.0,
-                         V.s, H.lv[0].x, H.omega, tid, nth, cs);
+        th_presmooth<Tr>(lv[0], Nz, V.r, V.v, -alpha, (const double*)nullptr, 0.0, V.s, H.omega, tl);
         if (!sync(TH_P_PRE_S)) return;
         if (!vcycle(V.s, V.sh)) return;
         // ---- t = op sh; (t, s), (t, t)
-        {
-            double acc[2] = {0.0, 0.0};
-            cells2([&](long long q, int i, int j, int kk) {
-                return make_double2(th_ax<Tr>(F0, Nz, V.sh, q, i, j, kk), V.s[q]);
-            }, [&](long long q, double2 a) {
-                V.t[q] = a.x;
-                acc[0] += a.x * a.y;
-                acc[1] += a.x * a.x;
-            });
-            block_sum<2>(acc, sm);
-            if (threadIdx.x == 0) { pB[2 * blockIdx.x] = acc[0]; pB[2 * blockIdx.x + 1] = acc[1]; }
-        }
-        if (!sync(TH_P_MATVEC_T)) return;
-        double ts[2];
-        sum_partials<2>(pB, G, 2, ts, sm);
-        omega = ts[1] > 0.0 ? ts[0] / ts[1] : 0.0;
+        acc[0] = acc[1] = 0.0;
+        cells2([&](unsigned q, int i, int j, int kk) {
+            return make_double2(th_ax<Tr>(F0, Nz, V.sh, q, i, j, kk), V.s[q]);
+        }, [&](unsigned q, double2 a) {
+            V.t[q] = a.x;
+            acc[0] += a.x * a.y;
+            acc[1] += a.x * a.x;
+        });
+        if (!reduce(TH_P_MATVEC_T, acc)) return;
+        omega = acc[1] > 0.0 ? acc[0] / acc[1] : 0.0;
         // ---- x += alpha ph + omega sh; r = s - omega t; (r, r), (rh, r)
-        {
-            double acc[2] = {0.0, 0.0};
-            cells2([&](long long q, int, int, int) {
-                return make_double3(V.x[q] + alpha * double(V.ph[q]) + omega * double(V.sh[q]), V.s[q] - omega * V.t[q],
-                                    V.rh[q]);
-            }, [&](long long q, double3 a) {
-                V.x[q] = a.x;
-                V.r[q] = a.y;
-                acc[0] += a.y * a.y;
-                acc[1] += a.z * a.y;
-            });
-            block_sum<2>(acc, sm);
-            if (threadIdx.x == 0) { pC[2 * blockIdx.x] = acc[0]; pC[2 * blockIdx.x + 1] = acc[1]; }
-        }
-        if (!sync(TH_P_UPDATE)) return;
-        sum_partials<2>(pC, G, 2, tot, sm);
-        res = sqrt(tot[0]) / bnorm;
+        acc[0] = acc[1] = 0.0;
+        cells2([&](unsigned q, int, int, int) {
+            return make_double3(V.x[q] + alpha * double(V.ph[q]) + omega * double(V.sh[q]), V.s[q] - omega * V.t[q],
+                                V.rh[q]);
+        }, [&](unsigned q, double3 a) {
+            V.x[q] = a.x;
+            V.r[q] = a.y;
+            acc[0] += a.y * a.y;
+            acc[1] += a.z * a.y;
+        });
+        if (!reduce(TH_P_UPDATE, acc)) return;
+        res = sqrt(acc[0]) / bnorm;
         rho = rho1;
-        rho1 = tot[1];
+        rho1 = acc[1];
         if (!(res == res)) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(&st->err, 0, (int)CP_ERR_NONFINITE);
+            if (team.lead()) atomicCAS(&st->err, 0, (int)CP_ERR_NONFINITE);
             return;
         }
         if (res <= rtol) { conv = true; ++it; break; }
         if (omega == 0.0) { ++it; break; }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (team.lead()) {
         st->iterations = it;
         st->converged = conv ? 1 : 0;
         st->residual = res;
@@ -888,7 +927,7 @@ using namespace cp;
 struct cp_thermal {
     cp_thermal_params prm{};
     ThK k{};
-    int dev = 0, numSMs = 0, grid = 0, gElem = 0;
+    int dev = 0, numSMs = 0, grid = 0, gElem = 0, threads = 256;   // grid, threads: the solver kernel's
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double *gamma = nullptr, *u = nullptr, *v = nullptr, *q0 = nullptr;
@@ -901,6 +940,7 @@ struct cp_thermal {
     // CP_PREC_MIXED: float copies of every level for the V-cycle, and the
     // preconditioned directions in float
     bool mixed = false;
+    size_t matSmem = 0;               // k_th_matrix's dynamic shared memory (bytes)
     std::vector<ThLevelT<float>> lvf;
     ThLevelT<float>* dlvf = nullptr;
     ThHierT<float> Hf{};
@@ -922,6 +962,14 @@ cp_status th_alloc(cp_thermal* t, T** p, size_t n) {
     TCK(cudaMemsetAsync(q, 0, std::max<size_t>(n, 1) * sizeof(T), t->stream));
     *p = static_cast<T*>(q);
     return CP_OK;
+}
+
+// the solver kernel of a context's size and precision
+template <bool Tr>
+const void* th_kernel(const cp_thermal* t) {
+    if (t->mixed)
+        return t->threads == 512 ? (const void*)k_th_bicgstab<Tr, float, 512> : (const void*)k_th_bicgstab<Tr, float, 256>;
+    return t->threads == 512 ? (const void*)k_th_bicgstab<Tr, double, 512> : (const void*)k_th_bicgstab<Tr, double, 256>;
 }
 
 // float copy of a level array (mixed precision)
@@ -962,22 +1010,24 @@ cp_status th_build_float_hierarchy(cp_thermal* t) {
     t->dlvf = static_cast<ThLevelT<float>*>(q);
     TCK(cudaMemcpyAsync(t->dlvf, t->lvf.data(), sizeof(ThLevelT<float>) * L, cudaMemcpyHostToDevice, t->stream));
     t->Hf.L = t->H.L;
-    t->Hf.cta = t->H.cta;
+    t->Hf.m = t->H.m;
     t->Hf.omega = t->H.omega;
     t->Hf.scale0 = t->H.scale0;
     t->Hf.scale = t->H.scale;
     t->Hf.lv = t->dlvf;
     t->Hf.prof = t->H.prof;
-    cp_status s = th_alloc(t, &t->phf, (size_t)t->k.n);
+    const size_t nm = (size_t)t->lv[t->H.m].n;
+    cp_status s = th_alloc(t, &t->Hf.bm, nm * nm);
+    if (s == CP_OK) s = th_alloc(t, &t->phf, (size_t)t->k.n);
     if (s != CP_OK) return s;
     return th_alloc(t, &t->shf, (size_t)t->k.n);
 }
 
 // Levels of 2 x 2 column aggregates down to a single column, all z-layers
-// kept; level 0 is the assembled system.  CP_TH_OMEGA, CP_TH_SCALE0,
-// CP_TH_SCALE and CP_TH_CTA_COLS override the smoothing weight, the
-// coarse-correction factors into level 0 and into the deeper levels, and the
-// size below which block 0 runs a level alone.
+// kept; level 0 is the assembled system.  From the first coarse level with at
+// most kThApply cells on the V-cycle is a matrix.  CP_TH_OMEGA, CP_TH_SCALE0
+// and CP_TH_SCALE override the smoothing weight and the coarse-correction
+// factors into level 0 and into the deeper levels.
 cp_status th_build_hierarchy(cp_thermal* t) {
     const ThK& k = t->k;
     ThLevel f0{};
@@ -1008,18 +1058,15 @@ cp_status th_build_hierarchy(cp_thermal* t) {
         t->lv.push_back(C);
     }
     const int L = (int)t->lv.size();
-    long long ctaCols = kThCtaCols;
-    if (const char* e = getenv("CP_TH_CTA_COLS")) ctaCols = std::max(atoll(e), 1LL);
-    int cta = L;
-    for (int l = 1; l < L; ++l)
-        if (t->lv[l].ncol <= ctaCols) { cta = l; break; }
+    int m = 1;
+    while (t->lv[m].n > kThApply) ++m;    // the last level is one column: Nz <= 16 cells
     void* q = nullptr;
     TCK(cudaMalloc(&q, sizeof(ThLevel) * L));
     t->allocs.push_back(q);
     t->dlv = static_cast<ThLevel*>(q);
     TCK(cudaMemcpyAsync(t->dlv, t->lv.data(), sizeof(ThLevel) * L, cudaMemcpyHostToDevice, t->stream));
     t->H.L = L;
-    t->H.cta = cta;
+    t->H.m = m;
     t->H.omega = kThOmega;
     t->H.scale0 = kThScale0;
     t->H.scale = kThScale;
@@ -1028,6 +1075,13 @@ cp_status th_build_hierarchy(cp_thermal* t) {
     if (const char* e = getenv("CP_TH_SCALE")) t->H.scale = atof(e);
     t->H.lv = t->dlv;
     t->H.prof = nullptr;
+    t->H.bm = nullptr;
+    t->matSmem = 0;
+    for (int l = m; l < L; ++l) t->matSmem += 3 * sizeof(double) * (size_t)t->lv[l].n;
+    if (!t->mixed) {
+        cp_status s = th_alloc(t, &t->H.bm, (size_t)t->lv[m].n * t->lv[m].n);
+        if (s != CP_OK) return s;
+    }
     if (getenv("CP_TH_PROFILE")) {
         TCK(cudaMalloc(&q, sizeof(unsigned long long) * TH_P_COUNT));
         t->allocs.push_back(q);
@@ -1043,14 +1097,14 @@ void th_print_profile(cp_thermal* t, bool Tr, int iters) {
     const double it = iters > 0 ? iters : 1;
     fprintf(stderr, "thermal %s profile, us per iteration (%d iterations):\n", Tr ? "adjoint" : "forward", iters);
     const char* top[] = {"init(total)", "update p + presmooth 0", "matvec v", "update s + presmooth 0", "matvec t",
-                         "update x, r", "block-0 levels"};
-    for (int i = 0; i <= TH_P_BLOCK0; ++i)
+                         "update x, r", "matrix level"};
+    for (int i = 0; i <= TH_P_APPLY; ++i)
         if (h[i]) fprintf(stderr, "  %-26s %9.1f\n", top[i], h[i] * 1e-3 / (i == TH_P_INIT ? 1.0 : it));
-    const char* kind[] = {"restrict from", "presmooth", "post residual", "post columns"};
-    for (int kd = 0; kd < 4; ++kd)
+    const char* kind[] = {"down from", "up into"};
+    for (int kd = 0; kd < 2; ++kd)
         for (int l = 0; l < 16; ++l) {
-            const unsigned long long v = h[TH_P_RESTRICT + 16 * kd + l];
-            if (v) fprintf(stderr, "  %-16s level %2d %9.1f\n", kind[kd], l, v * 1e-3 / it);
+            const unsigned long long v = h[TH_P_DOWN + 16 * kd + l];
+            if (v) fprintf(stderr, "  %-10s level %2d %9.1f\n", kind[kd], l, v * 1e-3 / it);
         }
 }
 
@@ -1090,16 +1144,27 @@ cp_status th_krylov(cp_thermal* t, const double* rhs, const ThVecs& V, ThStatus*
             if (s != CP_OK) return s;
         }
     }
+    // the matrix of the small levels, from the FP64 levels in either precision
+    {
+        const int g = (int)t->lv[t->H.m].n;
+        if (t->mixed)
+            k_th_matrix<Tr, float><<<g, kThMatThreads, t->matSmem, t->stream>>>(k.Nz, t->dlv, t->H.m, t->H.L, t->H.omega,
+                                                                               t->H.scale, t->Hf.bm);
+        else
+            k_th_matrix<Tr, double><<<g, kThMatThreads, t->matSmem, t->stream>>>(k.Nz, t->dlv, t->H.m, t->H.L,
+                                                                                t->H.omega, t->H.scale, t->H.bm);
+        TCK(cudaGetLastError());
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(t->grid);
-    cfg.blockDim = dim3(kThThreads);
+    cfg.blockDim = dim3(t->threads);
     cfg.stream = t->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cfg.dynamicSmemBytes = kThSmemBytes;
+    cfg.dynamicSmemBytes = 0;
     const ThVecsT<float> Vf{V.x, V.r, V.rh, V.p, V.v, V.s, V.t, t->phf, t->shf};
     const int rounds = t->mixed ? kThRefineRounds : 1;
     int total = 0;
@@ -1109,11 +1174,11 @@ cp_status th_krylov(cp_thermal* t, const double* rhs, const ThVecs& V, ThStatus*
         if (t->H.prof) TCK(cudaMemsetAsync(t->H.prof, 0, sizeof(unsigned long long) * TH_P_COUNT, t->stream));
         const int left = std::max(t->prm.maxiter - total, 0);
         if (t->mixed)
-            TCK(cudaLaunchKernelEx(&cfg, k_th_bicgstab<Tr, float>, k, t->lv[0], t->Hf, rhs, Vf, t->part, t->bar,
-                                   t->st, left, t->prm.rtol));
+            TCK(cudaLaunchKernelEx(&cfg, t->threads == 512 ? k_th_bicgstab<Tr, float, 512> : k_th_bicgstab<Tr, float, 256>,
+                                   k, t->lv[0], t->Hf, rhs, Vf, t->part, t->bar, t->st, left, t->prm.rtol));
         else
-            TCK(cudaLaunchKernelEx(&cfg, k_th_bicgstab<Tr, double>, k, t->lv[0], t->H, rhs, V, t->part, t->bar,
-                                   t->st, left, t->prm.rtol));
+            TCK(cudaLaunchKernelEx(&cfg, t->threads == 512 ? k_th_bicgstab<Tr, double, 512> : k_th_bicgstab<Tr, double, 256>,
+                                   k, t->lv[0], t->H, rhs, V, t->part, t->bar, t->st, left, t->prm.rtol));
         TCK(cudaEventRecord(t->ev1, t->stream));
         TCK(cudaMemcpyAsync(hs, t->st, sizeof *hs, cudaMemcpyDeviceToHost, t->stream));
         TCK(cudaStreamSynchronize(t->stream));
@@ -1216,18 +1281,21 @@ cp_status cp_thermal_create(const cp_thermal_params* p, cp_thermal** out) {
     // the forward and the adjoint kernel run on the same grid: every block resident
     // (the forward and adjoint kernels of the solve's precision)
     t->mixed = p->precision == CP_PREC_MIXED;
-    const void* kern[2] = {t->mixed ? (const void*)k_th_bicgstab<false, float> : (const void*)k_th_bicgstab<false, double>,
-                           t->mixed ? (const void*)k_th_bicgstab<true, float> : (const void*)k_th_bicgstab<true, double>};
+    t->threads = k.n >= kThLarge ? 512 : 256;
+    const void* kern[2] = {th_kernel<false>(t), th_kernel<true>(t)};
     int nb = 1 << 30;
     for (const void* f : kern) {
         int b = 0;
-        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kThSmemBytes) != cudaSuccess)
-            return bail(tfail(CP_ERR_CUDA, "the thermal solver kernel's shared memory (%zu bytes)", kThSmemBytes));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, kThThreads, kThSmemBytes);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, f, t->threads, 0);
         nb = std::min(nb, b);
     }
     if (nb < 1) return bail(tfail(CP_ERR_CUDA, "the thermal solver kernel does not fit on an SM"));
-    t->grid = t->numSMs * std::min(nb, 4);
+    t->grid = t->numSMs * std::min(nb, 2);
+    const void* mat[4] = {(const void*)k_th_matrix<false, double>, (const void*)k_th_matrix<true, double>,
+                          (const void*)k_th_matrix<false, float>, (const void*)k_th_matrix<true, float>};
+    for (const void* f : mat)
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kThMatSmemMax) != cudaSuccess)
+            return bail(tfail(CP_ERR_CUDA, "the thermal matrix kernel's shared memory (%zu bytes)", kThMatSmemMax));
     if ((s = th_build_hierarchy(t)) != CP_OK) return bail(s);
     if (t->mixed && (s = th_build_float_hierarchy(t)) != CP_OK) return bail(s);
     t->gElem = t->numSMs * 4;
