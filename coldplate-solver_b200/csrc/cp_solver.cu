@@ -26,6 +26,7 @@
 #include "cp_pcg.cuh"
 #include "cp_adjoint.cuh"
 #include "cp_batch.cuh"
+#include "cp_pool.cuh"
 
 using namespace cp;
 
@@ -145,7 +146,8 @@ struct cp_ctx {
     cudaGraphExec_t graph = nullptr;
     bool graphTried = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    std::vector<void*> allocs;
+    Arena mem;                         // every device array
+    PoolBlock stBlock, stageBlock;     // pinned: stHost, gammaStage
 };
 
 namespace {
@@ -153,17 +155,15 @@ namespace {
 template <typename T>
 cp_status dalloc(cp_ctx* c, T** ptr, size_t count) {
     void* q = nullptr;
-    CK(cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T)));
+    CK(c->mem.take(count * sizeof(T), &q));
     CK(cudaMemsetAsync(q, 0, std::max<size_t>(count, 1) * sizeof(T), c->stream));
-    c->allocs.push_back(q);
     *ptr = static_cast<T*>(q);
     return CP_OK;
 }
 
 cp_status dalloc_bytes(cp_ctx* c, void** ptr, size_t bytes) {
-    CK(cudaMalloc(ptr, std::max<size_t>(bytes, 1)));
+    CK(c->mem.take(bytes, ptr));
     CK(cudaMemsetAsync(*ptr, 0, std::max<size_t>(bytes, 1), c->stream));
-    c->allocs.push_back(*ptr);
     return CP_OK;
 }
 
@@ -930,7 +930,9 @@ cp_status cp_create(const cp_params* prm, cp_ctx** out) {
     c->histCap = prm->historyCapacity > 0 ? prm->historyCapacity : std::max(prm->maxIterations, 1);
     if ((s = dalloc(c, &c->hist, (size_t)c->histCap * kHistCols)) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->dpWin, (size_t)std::max(prm->dpConvergenceWindow, 1))) != CP_OK) return bail(s);
-    if (cudaMallocHost(&c->stHost, sizeof(Status)) != cudaSuccess) return bail(fail(CP_ERR_CUDA, "cudaMallocHost failed"));
+    if (host_cache().acquire(4096, &c->stBlock) != cudaSuccess) return bail(fail(CP_ERR_CUDA, "cudaMallocHost failed"));
+    static_assert(sizeof(Status) <= 4096, "the pinned status block");
+    c->stHost = static_cast<Status*>(c->stBlock.p);
     memset(c->stHost, 0, sizeof(Status));
     // all fluid until a geometry is set (SIMPLE.cpp:267-269)
     c->cellTypeHost.assign((size_t)M * N, 0.0);
@@ -939,6 +941,12 @@ cp_status cp_create(const cp_params* prm, cp_ctx** out) {
     if ((s = upload_cells(c, g.data())) != CP_OK) return bail(s);
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return bail(fail(CP_ERR_CUDA, "initialisation failed"));
     *out = c;
+    return CP_OK;
+}
+
+cp_status cp_release_cached_memory(void) {
+    device_cache().release_all();
+    host_cache().release_all();
     return CP_OK;
 }
 
@@ -958,9 +966,9 @@ cp_status cp_destroy(cp_ctx* c) {
         }
     }
     if (c->graph) cudaGraphExecDestroy(c->graph);
-    for (void* q : c->allocs) cudaFree(q);
-    if (c->stHost) cudaFreeHost(c->stHost);
-    if (c->gammaStage) cudaFreeHost(c->gammaStage);
+    c->mem.give_back();
+    host_cache().give(c->stBlock);
+    host_cache().give(c->stageBlock);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -983,10 +991,12 @@ static cp_status set_cells(cp_ctx* c, const double* src, long rows, long cols, l
             if (!std::isfinite(src[i * rs + j * cs])) return fail(CP_ERR_NONFINITE, "non-finite input at (%ld, %ld)", i, j);
     // gamma goes up from a pinned staging array the context keeps (DMA; no
     // fresh host pages per call)
-    if (!c->gammaStage && cudaMallocHost(&c->gammaStage, (size_t)M * N * sizeof(double)) != cudaSuccess) {
-        c->gammaStage = nullptr;
-        cudaGetLastError();
-        return fail(CP_ERR_CUDA, "cudaMallocHost of the gamma staging array failed");
+    if (!c->gammaStage) {
+        if (host_cache().acquire((size_t)M * N * sizeof(double), &c->stageBlock) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(CP_ERR_CUDA, "cudaMallocHost of the gamma staging array failed");
+        }
+        c->gammaStage = static_cast<double*>(c->stageBlock.p);
     }
     std::vector<double>& P = c->cellTypeHost;   // M x N padded; every entry is rewritten
     for (long i = 0; i < rows; ++i) {

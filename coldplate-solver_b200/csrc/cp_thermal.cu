@@ -40,6 +40,7 @@
 
 #include "../../include/cp_thermal.h"
 #include "cp_device.cuh"
+#include "cp_pool.cuh"
 
 // error string of the library (cp_solver.cu)
 cp_status cp_internal_set_error(cp_status s, const char* msg);
@@ -949,7 +950,7 @@ struct cp_thermal {
     unsigned* bar = nullptr;
     ThStatus* st = nullptr;
     bool hasInputs = false, solved = false;
-    std::vector<void*> allocs;
+    Arena mem;                        // every device array
 };
 
 namespace {
@@ -957,8 +958,7 @@ namespace {
 template <typename T>
 cp_status th_alloc(cp_thermal* t, T** p, size_t n) {
     void* q = nullptr;
-    TCK(cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T)));
-    t->allocs.push_back(q);
+    TCK(t->mem.take(n * sizeof(T), &q));
     TCK(cudaMemsetAsync(q, 0, std::max<size_t>(n, 1) * sizeof(T), t->stream));
     *p = static_cast<T*>(q);
     return CP_OK;
@@ -1005,8 +1005,7 @@ cp_status th_build_float_hierarchy(cp_thermal* t) {
         }
     }
     void* q = nullptr;
-    TCK(cudaMalloc(&q, sizeof(ThLevelT<float>) * L));
-    t->allocs.push_back(q);
+    TCK(t->mem.take(sizeof(ThLevelT<float>) * L, &q));
     t->dlvf = static_cast<ThLevelT<float>*>(q);
     TCK(cudaMemcpyAsync(t->dlvf, t->lvf.data(), sizeof(ThLevelT<float>) * L, cudaMemcpyHostToDevice, t->stream));
     t->Hf.L = t->H.L;
@@ -1061,8 +1060,7 @@ cp_status th_build_hierarchy(cp_thermal* t) {
     int m = 1;
     while (t->lv[m].n > kThApply) ++m;    // the last level is one column: Nz <= 16 cells
     void* q = nullptr;
-    TCK(cudaMalloc(&q, sizeof(ThLevel) * L));
-    t->allocs.push_back(q);
+    TCK(t->mem.take(sizeof(ThLevel) * L, &q));
     t->dlv = static_cast<ThLevel*>(q);
     TCK(cudaMemcpyAsync(t->dlv, t->lv.data(), sizeof(ThLevel) * L, cudaMemcpyHostToDevice, t->stream));
     t->H.L = L;
@@ -1083,8 +1081,7 @@ cp_status th_build_hierarchy(cp_thermal* t) {
         if (s != CP_OK) return s;
     }
     if (getenv("CP_TH_PROFILE")) {
-        TCK(cudaMalloc(&q, sizeof(unsigned long long) * TH_P_COUNT));
-        t->allocs.push_back(q);
+        TCK(t->mem.take(sizeof(unsigned long long) * TH_P_COUNT, &q));
         t->H.prof = static_cast<unsigned long long*>(q);
     }
     return CP_OK;
@@ -1301,11 +1298,9 @@ cp_status cp_thermal_create(const cp_thermal_params* p, cp_thermal** out) {
     t->gElem = t->numSMs * 4;
     if ((s = th_alloc(t, &t->part, (size_t)6 * kMaxBlocks)) != CP_OK) return bail(s);
     void* q = nullptr;
-    if (cudaMalloc(&q, 64) != cudaSuccess) return bail(tfail(CP_ERR_CUDA, "cudaMalloc"));
-    t->allocs.push_back(q);
+    if (t->mem.take(64, &q) != cudaSuccess) return bail(tfail(CP_ERR_CUDA, "cudaMalloc"));
     t->bar = static_cast<unsigned*>(q);
-    if (cudaMalloc(&q, sizeof(ThStatus)) != cudaSuccess) return bail(tfail(CP_ERR_CUDA, "cudaMalloc"));
-    t->allocs.push_back(q);
+    if (t->mem.take(sizeof(ThStatus), &q) != cudaSuccess) return bail(tfail(CP_ERR_CUDA, "cudaMalloc"));
     t->st = static_cast<ThStatus*>(q);
     if (cudaStreamSynchronize(t->stream) != cudaSuccess) return bail(tfail(CP_ERR_CUDA, "stream"));
     *out = t;
@@ -1315,7 +1310,7 @@ cp_status cp_thermal_create(const cp_thermal_params* p, cp_thermal** out) {
 cp_status cp_thermal_destroy(cp_thermal* t) {
     if (!t) return CP_OK;
     if (t->stream) cudaStreamSynchronize(t->stream);
-    for (void* q : t->allocs) cudaFree(q);
+    t->mem.give_back();
     if (t->ev0) cudaEventDestroy(t->ev0);
     if (t->ev1) cudaEventDestroy(t->ev1);
     if (t->stream) cudaStreamDestroy(t->stream);

@@ -173,13 +173,18 @@ cp_status cp_read_fluid_params(const char* path, cp_params* p);
  * and gamma at 1 (all fluid), like SIMPLE::initializeMemory. */
 cp_status cp_create(const cp_params* p, cp_ctx** out);
 cp_status cp_destroy(cp_ctx* ctx);
+/* The memory of destroyed contexts (and thermal contexts) is kept for the next
+ * ones, at most 4 GB of device and 256 MB of pinned host memory a CUDA
+ * context.  It is given back when an allocation fails, at exit, and by this
+ * call (for the current device). */
+cp_status cp_release_cached_memory(void);
 
 /* Geometry.  cellType: Ny x Nx, 0 fluid .. 1 solid (geometry_fluid.txt,
  * SIMPLE.cpp:633-690, converted as SIMPLE.cpp:695-777).  gamma: Ny x Nx
  * density, 1 fluid .. 0 solid (set directly, e.g. by an optimiser).  A
  * non-finite entry returns CP_ERR_NONFINITE and leaves the geometry as it
  * was.  The first call allocates a pinned (M x N doubles) staging array that
- * the context keeps for later calls and frees in cp_destroy. */
+ * the context keeps for later calls and gives up in cp_destroy. */
 cp_status cp_set_cell_type(cp_ctx* ctx, const double* cellType, long rows, long cols,
                            long row_stride, long col_stride);
 cp_status cp_set_gamma(cp_ctx* ctx, const double* gamma, long rows, long cols,
