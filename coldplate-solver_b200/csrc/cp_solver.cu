@@ -1309,6 +1309,22 @@ cp_status adjoint_sweeps(cp_ctx* c, const KParams& k, const MomSys<double>& S, c
     return CP_OK;
 }
 
+// the Gram-Schmidt kernels at nv rounded up to a multiple of 8 (nv <= 32)
+void kry_mdot(int nb, cudaStream_t s, const double* w, const double* B, size_t L, int nv, double* part) {
+    static_assert(kKryMaxDots == 32, "four instances");
+    if (nv <= 8) k_kry_mdot<8><<<nb, 256, 0, s>>>(w, B, L, nv, part);
+    else if (nv <= 16) k_kry_mdot<16><<<nb, 256, 0, s>>>(w, B, L, nv, part);
+    else if (nv <= 24) k_kry_mdot<24><<<nb, 256, 0, s>>>(w, B, L, nv, part);
+    else k_kry_mdot<32><<<nb, 256, 0, s>>>(w, B, L, nv, part);
+}
+template <bool Self>
+void kry_axpy_mdot(int nb, cudaStream_t s, double* w, const double* B, size_t L, int nv, const double* h, double* part) {
+    if (nv <= 8) k_kry_axpy_mdot<8, Self><<<nb, 256, 0, s>>>(w, B, L, nv, h, -1.0, part);
+    else if (nv <= 16) k_kry_axpy_mdot<16, Self><<<nb, 256, 0, s>>>(w, B, L, nv, h, -1.0, part);
+    else if (nv <= 24) k_kry_axpy_mdot<24, Self><<<nb, 256, 0, s>>>(w, B, L, nv, h, -1.0, part);
+    else k_kry_axpy_mdot<32, Self><<<nb, 256, 0, s>>>(w, B, L, nv, h, -1.0, part);
+}
+
 template <typename TV>
 cp_status adjoint_prhs(cp_ctx* c, const KParams& k, const double* du, const double* dv, const double* rp) {
     PcgBufs<TV> B = pcg_bufs<TV>(c);
@@ -1513,7 +1529,7 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
     };
     // h[0..nv) = <w, B_0..B_nv-1> into dst (device)
     auto mdot = [&](const double* w, const double* B, int nv, double* dst) -> cp_status {
-        k_kry_mdot<<<nb, 256, 0, c->stream>>>(w, B, L, nv, c->adjKryPart);
+        kry_mdot(nb, c->stream, w, B, L, nv, c->adjKryPart);
         CK(cudaGetLastError());
         k_kry_sum<<<1, 1024, 0, c->stream>>>(c->adjKryPart, nb, nv, dst);
         CK(cudaGetLastError());
@@ -1565,11 +1581,11 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
             double* nr = c->adjH + 2 * kKryMaxDots;
             // (each projection fused with the dot products that follow it)
             if ((s = mdot(W, Vq(0), j + 1, h1)) != CP_OK) return s;
-            k_kry_axpy_mdot<<<nb, 256, 0, c->stream>>>(W, Vq(0), L, j + 1, h1, -1.0, j + 1, 0, c->adjKryPart);
+            kry_axpy_mdot<false>(nb, c->stream, W, Vq(0), L, j + 1, h1, c->adjKryPart);
             CK(cudaGetLastError());
             k_kry_sum<<<1, 1024, 0, c->stream>>>(c->adjKryPart, nb, j + 1, h2);
             CK(cudaGetLastError());
-            k_kry_axpy_mdot<<<nb, 256, 0, c->stream>>>(W, Vq(0), L, j + 1, h2, -1.0, 1, 1, c->adjKryPart);
+            kry_axpy_mdot<true>(nb, c->stream, W, Vq(0), L, j + 1, h2, c->adjKryPart);
             CK(cudaGetLastError());
             k_kry_sum<<<1, 1024, 0, c->stream>>>(c->adjKryPart, nb, 1, nr);
             CK(cudaGetLastError());
