@@ -716,7 +716,7 @@ __device__ __forceinline__ bool team_outer(const Team& T, unsigned& target, cons
     // ---- k_mass, then the smoothed-aggregation PCG (k_pcg_sa)
     mass_pass<TC>(k, f.u, f.v, f.uStar, f.vStar, f.B.rhs, tid, nth, f.partM + (size_t)T.rank * 4);
     if (!team_sync(T, target)) return false;
-    if (!pcg_sa<TC>(T, target, k, st, f.dE, f.dN, f.B, f.H, f.pStar, f.partP)) return false;
+    if (!pcg_sa<TC, true>(T, target, k, st, f.dE, f.dN, f.B, f.H, f.pStar, f.partP)) return false;
     if (!team_sync(T, target)) return false;
     // ---- k_correct (iterations.cpp:556-597), k_bc, k_finalize
     correct_cells(k, iter, f.u, f.v, f.p, f.uStar, f.vStar, f.pStar, f.dE, f.dN, tid, nth);

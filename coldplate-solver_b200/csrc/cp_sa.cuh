@@ -538,6 +538,131 @@ __device__ __forceinline__ void sa_up(const Team& T, const SaLevel<TV>& f, const
     }
 }
 
+// The two transfers as marches over rows, for teams of a few CTAs (batches),
+// whose warps each have many rows of a level: t of a row is formed once instead
+// of 5/3 times and three times, and what a team is short of is instructions, not
+// loads in flight.  24 batched fields, 20 iterations: 156 ms with the steps
+// above, 140 with these.  On the whole grid the steps are the faster ones
+// (level 1 of 2048 x 1024 excepted, and there the registers of both forms
+// together cost more in the passes over level 0 than the march saves).
+template <typename TV>
+__device__ __forceinline__ void sa_down_march(const Team& T, const SaLevel<TV>& f, const SaLevel<TV>& C, double om, bool last) {
+    const int lane = threadIdx.x & 31, nw = T.nth() >> 5;
+    const SaRuns W((C.nJ + 8) / 9, C.nI, nw);
+    for (int c = sa_task(T, W.n, nw); c < W.n; c += nw) {
+        const int s = c % W.S, I0 = 1 + (c / W.S) * W.R, I1 = min(C.nI, I0 + W.R - 1);
+        const int col = 27 * s - 1 + lane;
+        const bool act = col >= 1 && col <= f.nJ;
+        const int J = 9 * s + 1 + lane;
+        const bool out = lane < 9 && J <= C.nJ;
+        auto ldx = [&](int r) -> TV { return act && r >= 1 && r <= f.nI ? f.x[(size_t)r * f.P + col] : (TV)0; };
+        const int rb = 3 * I0 - 3, re = 3 * I1 + 1;
+        SaTriple<TV> xs = sa_triple(ldx(rb - 1)), xc = sa_triple(ldx(rb));
+        // the ring row above waits for the emission, where its terms come after
+        // the own rows' as in sa_down: the same sums to the last bit
+        double vO = 0.0, vH = 0.0, tA = 0.0, tR = 0.0;
+        TV pA[2] = {(TV)0, (TV)0}, pR[2] = {(TV)0, (TV)0};
+        int role = 2, I = I0 - 1;
+        for (int r = rb; r <= re; ++r) {
+            const bool in = act && r >= 1 && r <= f.nI;
+            const size_t q = (size_t)r * f.P + col;
+            TV a[9], b = (TV)0, p[4];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) a[k] = in ? f.c[k][q] : (TV)0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) p[k] = in ? f.pw[k][q] : (TV)0;
+            if (in) b = f.b[q];
+            TV d = (TV)1;
+            if (role == 0 && out && !last && I >= I0) d = C.c[4][(size_t)I * C.P + J];
+            const SaTriple<TV> xn = sa_triple(ldx(r + 1));
+            const double t = (double)b - sa_dot9(a, xs, xc, xn);
+            xs = xc;
+            xc = xn;
+            if (role == 0) {
+                // the ring row below the previous aggregate completes it
+                vO += (double)pR[0] * tR;
+                vH += (double)pR[1] * tR;
+                vO += (double)p[2] * t;
+                vH += (double)p[3] * t;
+                const double h0 = __shfl_sync(0xffffffffu, vH, 3 * lane + 1), o1 = __shfl_sync(0xffffffffu, vO, 3 * lane + 2),
+                             o2 = __shfl_sync(0xffffffffu, vO, 3 * lane + 3), o3 = __shfl_sync(0xffffffffu, vO, 3 * lane + 4),
+                             h4 = __shfl_sync(0xffffffffu, vH, 3 * lane + 5);
+                if (I >= I0 && out) {
+                    const double v = ((h0 + o1) + (o2 + o3)) + h4;
+                    const size_t qc = (size_t)I * C.P + J;
+                    C.b[qc] = (TV)v;
+                    if (!last) C.x[qc] = (TV)(om * v / (double)d);
+                }
+                ++I;
+                vO = vH = 0.0;
+                tR = tA;
+                pR[0] = pA[0];
+                pR[1] = pA[1];
+            }
+            vO += (double)p[0] * t;
+            vH += (double)p[1] * t;
+            tA = t;
+            pA[0] = p[2];
+            pA[1] = p[3];
+            role = role == 2 ? 0 : role + 1;
+        }
+    }
+}
+
+template <typename TV>
+__device__ __forceinline__ void sa_up_march(const Team& T, const SaLevel<TV>& f, const SaLevel<TV>& C, double om) {
+    const int lane = threadIdx.x & 31, nw = T.nth() >> 5;
+    const SaRuns W((f.nJ + 29) / 30, f.nI, nw);
+    const TV* e = C.y;
+    for (int c = sa_task(T, W.n, nw); c < W.n; c += nw) {
+        const int s = c % W.S, i0 = 1 + (c / W.S) * W.R, i1 = min(f.nI, i0 + W.R - 1);
+        const int col = 30 * s + lane;
+        const bool act = col >= 1 && col <= f.nJ, own = act && lane >= 1 && lane <= 30;
+        const int J = act ? (col - 1) / 3 + 1 : 0, Jh = act ? J + sa_side(col) : 0;
+        auto ldO = [&](int I) -> TV { return e[(size_t)I * C.P + J]; };
+        auto ldH = [&](int I) -> TV { return e[(size_t)I * C.P + Jh]; };
+        const int rb = max(i0 - 1, 1), re = i1 + 1;
+        int I = (rb - 1) / 3 + 1, role = (rb - 1) % 3;
+        TV oP = ldO(I - 1), hP = ldH(I - 1), oC = ldO(I), hC = ldH(I), oN = ldO(I + 1), hN = ldH(I + 1);
+        SaTriple<double> ts = {0.0, 0.0, 0.0}, tc = ts;
+        for (int r = rb; r <= re; ++r) {
+            // y of row r - 1 needs its operator row; loaded with row r's weights
+            const int ry = r - 1;
+            const bool yr = own && ry >= i0;
+            const size_t q = (size_t)r * f.P + col, qy = q - f.P;
+            const bool in = act && r <= f.nI;
+            TV a[9], b = (TV)0, p[4], x = (TV)0;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) a[k] = yr ? f.c[k][qy] : (TV)0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) p[k] = in ? f.pw[k][q] : (TV)0;
+            if (yr) b = f.b[qy];
+            if (in) x = f.x[q];
+            const TV oV = role == 0 ? oP : oN, hV = role == 0 ? hP : hN;
+            double t = (double)x;
+            t += (double)p[0] * (double)oC;
+            t += (double)p[1] * (double)hC;
+            if (role != 1) {
+                t += (double)p[2] * (double)oV;
+                t += (double)p[3] * (double)hV;
+            }
+            const SaTriple<double> tn = sa_triple(t);
+            if (yr) {
+                f.y[qy] = (TV)(tc.c + om * ((double)b - sa_dot9(a, ts, tc, tn)) / (double)a[4]);
+            }
+            ts = tc;
+            tc = tn;
+            if (++role == 3) {
+                role = 0;
+                ++I;
+                oP = oC; hP = hC;
+                oC = oN; hC = hN;
+                if (r < re && I + 1 <= C.nI + 1) { oN = ldO(I + 1); hN = ldH(I + 1); }
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------------------- level 0
 // Level 0's operator: face coefficients fE (east), fN (north), the diagonal
 // d and its inverse.  Every level-0 array is zero on the frame (only the
@@ -1104,10 +1229,10 @@ __device__ __forceinline__ double sa0_up(const Team& T, const Sa0<TV>& A, const 
 
 // ---------------------------------------------------------------- the solver
 // The PCG of one pressure-correction solve on a team of CTAs (the whole grid
-// in k_pcg_sa, a group of CTAs in the batched kernel); returns false if a
+// in k_pcg_sa; Few: a group of CTAs in the batched kernel); returns false if a
 // barrier gave up.  Ends without a barrier after writing p'.  part: at least
 // 4 doubles a CTA.
-template <typename TV>
+template <typename TV, bool Few>
 __device__ __forceinline__ bool pcg_sa(const Team& T, unsigned& target, const KParams& k, Status* st,
                                        const double* dE, const double* dN, const PcgBufs<TV>& B,
                                        const SaHier<TV>& H, double* pStar, double* part) {
@@ -1208,7 +1333,8 @@ __device__ __forceinline__ bool pcg_sa(const Team& T, unsigned& target, const KP
     // ---- the V-cycle below level 0 and the ascent into it: z = M b
     auto vcycle = [&](const TV* b, double& rz) __attribute__((always_inline)) -> bool {
         for (int l = 1; l < H.Ld; ++l) {
-            sa_down(T, H.lv[l], H.lv[l + 1], om, l + 1 == H.Ld);
+            if constexpr (Few) sa_down_march(T, H.lv[l], H.lv[l + 1], om, l + 1 == H.Ld);
+            else sa_down(T, H.lv[l], H.lv[l + 1], om, l + 1 == H.Ld);
             if (!team_sync(T, target)) return false;
             tick(SA_P_DOWN + l);
         }
@@ -1216,7 +1342,8 @@ __device__ __forceinline__ bool pcg_sa(const Team& T, unsigned& target, const KP
         if (!team_sync(T, target)) return false;
         tick(SA_P_DENSE);
         for (int l = H.Ld - 1; l >= 1; --l) {
-            sa_up(T, H.lv[l], H.lv[l + 1], om);
+            if constexpr (Few) sa_up_march(T, H.lv[l], H.lv[l + 1], om);
+            else sa_up(T, H.lv[l], H.lv[l + 1], om);
             if (!team_sync(T, target)) return false;
             tick(SA_P_UP + l);
         }
@@ -1282,7 +1409,7 @@ __global__ void __launch_bounds__(512, 1) k_pcg_sa(KParams k, Status* st, const 
                                                 unsigned* bar) {
     if (st->done) return;
     unsigned target = 0;
-    pcg_sa<TV>(grid_team(bar, &st->err), target, k, st, dE, dN, B, H, pStar, part);
+    pcg_sa<TV, false>(grid_team(bar, &st->err), target, k, st, dE, dN, B, H, pStar, part);
 }
 
 }  // namespace cp
