@@ -696,9 +696,10 @@ __device__ __forceinline__ bool team_outer(const Team& T, unsigned& target, cons
         if (!jacobi_component<TC, Mixed, true>(k, f.U, f.u, f.xU0, f.xU1, f.partJ, T, target, curU, itU)) return false;
         if (!jacobi_component<TC, Mixed, false>(k, f.V, f.v, f.xV0, f.xV1, f.partJ, T, target, curV, itV)) return false;
         double mu = jacobi_scatter<TC, Mixed, true>(k, f.u, curU < 0 ? nullptr : (curU ? f.xU1 : f.xU0), f.uStar,
-                                                    maxVel, tid, nth);
+                                                    maxVel, true, tid, nth);
         double mv = jacobi_scatter<TC, Mixed, false>(k, f.v, curV < 0 ? nullptr : (curV ? f.xV1 : f.xV0), f.vStar,
-                                                     maxVel, tid, nth);
+                                                     maxVel, true, tid, nth);
+        apply_bc_const(k, iter, f.uStar, f.vStar, f.gamma, tid, nth);
         mu = warp_max(mu);
         mv = warp_max(mv);
         if ((threadIdx.x & 31) == 0) {
@@ -709,8 +710,6 @@ __device__ __forceinline__ bool team_outer(const Team& T, unsigned& target, cons
             st->itersU = itU;
             st->itersV = itV;
         }
-        if (!team_sync(T, target)) return false;
-        apply_bc(k, iter, f.uStar, f.vStar, nullptr, f.gamma, tid, nth);
     }
     if (!team_sync(T, target)) return false;
     // ---- k_mass, then the smoothed-aggregation PCG (k_pcg_sa)
@@ -720,8 +719,6 @@ __device__ __forceinline__ bool team_outer(const Team& T, unsigned& target, cons
     if (!team_sync(T, target)) return false;
     // ---- k_correct (iterations.cpp:556-597), k_bc, k_finalize
     correct_cells(k, iter, f.u, f.v, f.p, f.uStar, f.vStar, f.pStar, f.dE, f.dN, tid, nth);
-    if (!team_sync(T, target)) return false;
-    apply_bc(k, iter, f.u, f.v, f.p, f.gamma, tid, nth);
     if (!team_sync(T, target)) return false;
     if (T.rank == 0) {
         const FinalizeArgs fa{f.u, f.v, f.p, f.gamma, f.partM, T.size, f.hist, f.histCap, f.dpWin};

@@ -79,12 +79,34 @@ __device__ __forceinline__ void apply_bc(const KParams& k, int iter, double* u, 
     }
 }
 
-__global__ void k_bc(KParams k, Status* st, double* u, double* v, double* p, const double* gamma, int resetMax) {
+// The velocity BCs that do not copy an interior value (inlet, walls).  The rest
+// (the outlet's u and v, the pressure frame) follow an interior value each, and
+// the passes that write that value write them with it.
+__device__ __forceinline__ void apply_bc_const(const KParams& k, int iter, double* u, double* v, const double* gamma,
+                                               int t0, int stride) {
+    const Dims d = k.d;
+    const int M = d.M, N = d.N;
+    const double Uin = inlet_velocity(k, iter);
+    const int L = (M > N ? M : N) + 1;
+    for (int t = t0; t < L; t += stride) {
+        if (t <= M) u[at(d, t, 0)] = inlet_fluid(k, gamma, t) ? Uin : 0.0;
+        if (t >= 1 && t <= N - 1) { u[at(d, 0, t)] = 0.0; u[at(d, M, t)] = 0.0; }
+        if (t <= N) { v[at(d, 0, t)] = 0.0; v[at(d, M - 1, t)] = 0.0; }
+        if (t >= 1 && t <= M - 2) v[at(d, t, 0)] = 0.0;
+    }
+}
+
+// The BCs before an iteration; block 0 also clears the iteration's max-change
+// counters and the barrier counters of the persistent kernels behind it
+__global__ void k_bc(KParams k, Status* st, double* u, double* v, double* p, const double* gamma, unsigned* barJ,
+                     unsigned* barP) {
     if (st->done) return;
     const int iter = st->iter;
-    if (resetMax && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         st->maxDU = 0ull;
         st->maxDV = 0ull;
+        *barJ = 0u;
+        *barP = 0u;
     }
     apply_bc(k, iter, u, v, p, gamma, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
@@ -491,10 +513,11 @@ __device__ __forceinline__ bool jacobi_component(const KParams& k, const MomSys<
     return true;
 }
 
-// scatter with clamp and max |u* - u| (momentum_solver.cpp:335-351)
+// scatter with clamp and max |u* - u| (momentum_solver.cpp:335-351); with
+// outlet, the outlet column (boundaries.cpp:50-118) as a copy of the last one
 template <typename TC, bool Mixed, bool IsU>
 __device__ __forceinline__ double jacobi_scatter(const KParams& k, const double* field, const TC* xr,
-                                                 double* out, double maxVel, int tid, int nth) {
+                                                 double* out, double maxVel, bool outlet, int tid, int nth) {
     const Dims d = k.d;
     int i1, j1;
     mom_range<IsU>(d, i1, j1);
@@ -508,6 +531,7 @@ __device__ __forceinline__ double jacobi_scatter(const KParams& k, const double*
         const double nv = dclamp(xv, -maxVel, maxVel);
         m = dmax(m, fabs(nv - field[c]));
         out[c] = nv;
+        if (outlet && j == j1) out[c + 1] = nv;
     }
     return m;
 }
@@ -539,8 +563,9 @@ __global__ void __launch_bounds__(Seq ? kJacSegThreads : kJacThreads, Seq ? 3 : 
             return;
     }
     double mu = 0.0, mv = 0.0;
-    if (doU) mu = jacobi_scatter<TC, Mixed, true>(k, u, curU < 0 ? nullptr : (curU ? xU1 : xU0), out.uStar, maxVel, tid, nth);
-    if (doV) mv = jacobi_scatter<TC, Mixed, false>(k, v, curV < 0 ? nullptr : (curV ? xV1 : xV0), out.vStar, maxVel, tid, nth);
+    if (doU) mu = jacobi_scatter<TC, Mixed, true>(k, u, curU < 0 ? nullptr : (curU ? xU1 : xU0), out.uStar, maxVel, applyBC, tid, nth);
+    if (doV) mv = jacobi_scatter<TC, Mixed, false>(k, v, curV < 0 ? nullptr : (curV ? xV1 : xV0), out.vStar, maxVel, applyBC, tid, nth);
+    if (applyBC) apply_bc_const(k, iter, out.uStar, out.vStar, gamma, tid, nth);
     mu = warp_max(mu);
     mv = warp_max(mv);
     if ((threadIdx.x & 31) == 0) {
@@ -550,11 +575,6 @@ __global__ void __launch_bounds__(Seq ? kJacSegThreads : kJacThreads, Seq ? 3 : 
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (doU) st->itersU = itU;
         if (doV) st->itersV = itV;
-    }
-    if (applyBC) {
-        target += G;
-        if (!grid_barrier(bar, target, &st->err)) return;
-        apply_bc(k, iter, out.uStar, out.vStar, nullptr, gamma, tid, nth);
     }
 }
 
@@ -614,7 +634,10 @@ __global__ void k_mass(KParams k, const Status* st, const double* u, const doubl
 
 // ------------------------------------------------------------------ correction
 // p += pAlpha p' on [1,M-1] x [1,N-1]; u = clamp(u* + clamp(dE (p'_ij - p'_i,j+1)))
-// on U unknowns and the same for v (iterations.cpp:558-597).
+// on U unknowns and the same for v (iterations.cpp:558-597); then the boundary
+// conditions (iterations.cpp:567, 599), each by the thread that owns the
+// interior value it copies.  The inlet and the walls have their values from the
+// start of the iteration.
 __device__ __forceinline__ void correct_cells(const KParams& k, int iter, double* u, double* v, double* p,
                                               const double* uStar, const double* vStar, const double* pStar,
                                               const double* dE, const double* dN, int tid, int nth) {
@@ -626,18 +649,25 @@ __device__ __forceinline__ void correct_cells(const KParams& k, int iter, double
         const int i = 1 + t / w, j = 1 + t % w;
         const size_t c = at(d, i, j);
         const double ps = pStar[c];
-        p[c] += k.pAlpha * ps;
+        const double np = p[c] + k.pAlpha * ps;
+        p[c] = np;
+        if (i == 1) p[at(d, 0, j)] = np;
+        if (i == M - 1) p[at(d, M, j)] = np;
+        if (j == 1) p[at(d, i, 0)] = np;
+        if (j == w) p[c + 1] = 0.0;
         if (j <= N - 2) {
             double du = dE[c] * (ps - pStar[c + 1]);
             du = dmax(-maxVel, dmin(maxVel, du));
-            const double nu = uStar[c] + du;
-            u[c] = dmax(-maxVel, dmin(maxVel, nu));
+            const double nu = dmax(-maxVel, dmin(maxVel, uStar[c] + du));
+            u[c] = nu;
+            if (j == N - 2) u[c + 1] = nu;
         }
         if (i <= M - 2) {
             double dv = dN[c] * (ps - pStar[c + d.P]);
             dv = dmax(-maxVel, dmin(maxVel, dv));
-            const double nv = vStar[c] + dv;
-            v[c] = dmax(-maxVel, dmin(maxVel, nv));
+            const double nv = dmax(-maxVel, dmin(maxVel, vStar[c] + dv));
+            v[c] = nv;
+            if (j == w) v[c + 1] = nv;
         }
     }
 }
@@ -662,14 +692,15 @@ __device__ void finish_metrics(double area, double fs, double st, double dy, dou
 }
 
 // kind 0: plane at x (interpolated), 1: inlet patch, 2: outlet patch
-__device__ void sample_metric(const KParams& k, const double* u, const double* v, const double* p,
-                              const double* gamma, int kind, double x, double* m, double* sm) {
+// one thread's share of the sample, rows 1 + t, 1 + t + nt, ...: acc[5] = {area,
+// flux, static, dynamic, flux-weighted total}
+__device__ __forceinline__ void sample_rows(const KParams& k, const double* u, const double* v, const double* p,
+                                            const double* gamma, int kind, double x, int t, int nt, double (&acc)[5]) {
     const Dims d = k.d;
     const int M = d.M, N = d.N, NC = N - 1;
     const double hx = k.hx, hy = k.hy, rho = k.rho;
-    double acc[5] = {0, 0, 0, 0, 0};  // area, flux, static, dyn, totalWeighted
     int cl = 0, cr = 0;
-    double t = 0.0;
+    double wt = 0.0;
     if (kind == 0 && NC > 1) {
         const double xMin = 0.5 * hx, xMax = ((double)NC - 0.5) * hx;
         const double xc = dmax(xMin, dmin(x, xMax));
@@ -678,10 +709,10 @@ __device__ void sample_metric(const KParams& k, const double* u, const double* v
         if (cl < 0) cl = 0;
         cr = cl + 1;
         const double xl = ((double)cl + 0.5) * hx, xr = ((double)cr + 0.5) * hx;
-        t = (fabs(xr - xl) < 1e-12) ? 0.0 : (xc - xl) / (xr - xl);
-        t = dmax(0.0, dmin(1.0, t));
+        wt = (fabs(xr - xl) < 1e-12) ? 0.0 : (xc - xl) / (xr - xl);
+        wt = dmax(0.0, dmin(1.0, wt));
     }
-    for (int i = 1 + threadIdx.x; i < M; i += blockDim.x) {
+    for (int i = 1 + t; i < M; i += nt) {
         const int row = i - 1;
         const int vt = (i - 1 < M - 1) ? i - 1 : M - 1, vb = (i < M - 1) ? i : M - 1;
         double staticP, un, vtan;
@@ -689,12 +720,12 @@ __device__ void sample_metric(const KParams& k, const double* u, const double* v
             if (cl < 0 || cl >= NC || cr < 0 || cr >= NC) continue;
             if (gamma[at(d, row, cl)] < 1.0 - 1e-6 || gamma[at(d, row, cr)] < 1.0 - 1e-6) continue;
             const int pl = cl + 1 < N ? cl + 1 : N, pr = cr + 1 < N ? cr + 1 : N;
-            staticP = (1.0 - t) * p[at(d, i, pl)] + t * p[at(d, i, pr)];
+            staticP = (1.0 - wt) * p[at(d, i, pl)] + wt * p[at(d, i, pr)];
             const int ul = cl < N - 1 ? cl : N - 1, ur = cr < N - 1 ? cr : N - 1;
-            un = (1.0 - t) * u[at(d, i, ul)] + t * u[at(d, i, ur)];
+            un = (1.0 - wt) * u[at(d, i, ul)] + wt * u[at(d, i, ur)];
             const int vl = cl < N ? cl : N, vr = cr < N ? cr : N;
-            const double vTop = (1.0 - t) * v[at(d, vt, vl)] + t * v[at(d, vt, vr)];
-            const double vBot = (1.0 - t) * v[at(d, vb, vl)] + t * v[at(d, vb, vr)];
+            const double vTop = (1.0 - wt) * v[at(d, vt, vl)] + wt * v[at(d, vt, vr)];
+            const double vBot = (1.0 - wt) * v[at(d, vb, vl)] + wt * v[at(d, vb, vr)];
             vtan = 0.5 * (vTop + vBot);
         } else {
             const bool inlet = (kind == 1);
@@ -715,8 +746,6 @@ __device__ void sample_metric(const KParams& k, const double* u, const double* v
         const double fa = fabs(rho * un * hy);
         if (fa > 0.0) { acc[1] += fa; acc[4] += tot * fa; }
     }
-    block_sum<5>(acc, sm);
-    finish_metrics(acc[0], acc[1], acc[2], acc[3], acc[4], m);
 }
 
 struct FinalizeArgs {
@@ -729,42 +758,51 @@ struct FinalizeArgs {
 };
 
 // One block: residual norms from the k_mass partials, the four pressure
-// samples, the history row and the stop rules of one field.
+// samples, the history row and the stop rules of one field.  Everything it
+// reads is in flight at once (a quarter of the block a sample) and summed
+// behind one block barrier; a sample after the other took 21 us at 253 x 127
+// and 29 us at 2048 x 1024, launch included, now 13 and 19.  At least 128 threads, a multiple of 128.
 __device__ __forceinline__ void finalize_block(const KParams& k, Status* st, const FinalizeArgs& a) {
-    __shared__ double sm[32 * 5];
+    __shared__ double sm[32][9];
     __shared__ double met[4][5];
-    double sums[4];
+    __shared__ double sums[4];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     {
-        double s4[4] = {0, 0, 0, 0};
-        double mx = 0.0;
+        // {sum du^2, sum dv^2, sum b^2, max |b|} and the warp's sample
+        double r[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         for (int b = threadIdx.x; b < a.nbM; b += blockDim.x) {
-            s4[0] += a.partM[b * 4 + 0];
-            s4[1] += a.partM[b * 4 + 1];
-            s4[2] += a.partM[b * 4 + 2];
-            mx = dmax(mx, a.partM[b * 4 + 3]);
+            r[0] += a.partM[b * 4 + 0];
+            r[1] += a.partM[b * 4 + 1];
+            r[2] += a.partM[b * 4 + 2];
+            r[3] = dmax(r[3], a.partM[b * 4 + 3]);
         }
-        s4[3] = 0.0;
-        double s3[3] = {s4[0], s4[1], s4[2]};
-        block_sum<3>(s3, sm);
-        mx = warp_max(mx);
+        const int nt = blockDim.x >> 2, q = threadIdx.x / nt;
+        double acc[5] = {0, 0, 0, 0, 0};
+        sample_rows(k, a.u, a.v, a.p, a.gamma, q < 2 ? 0 : q - 1, q == 0 ? k.xCoreIn : k.xCoreOut, threadIdx.x - q * nt, nt, acc);
+#pragma unroll
+        for (int e = 0; e < 5; ++e) r[4 + e] = acc[e];
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+            r[e] = e == 3 ? warp_max(r[e]) : warp_sum(r[e]);
+            if (lane == 0) sm[wid][e] = r[e];
+        }
         __syncthreads();
-        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mx;
+        if (threadIdx.x < 4) {
+            double t = 0.0;
+            for (int w = 0; w < nw; ++w) t = threadIdx.x == 3 ? dmax(t, sm[w][3]) : t + sm[w][threadIdx.x];
+            sums[threadIdx.x] = t;
+        } else if (threadIdx.x >= 32 && threadIdx.x < 36) {
+            const int s = threadIdx.x - 32, w0 = s * (nw >> 2);
+            double t[5] = {0, 0, 0, 0, 0};
+            for (int w = w0; w < w0 + (nw >> 2); ++w)
+#pragma unroll
+                for (int e = 0; e < 5; ++e) t[e] += sm[w][4 + e];
+            double m[5];
+            finish_metrics(t[0], t[1], t[2], t[3], t[4], m);
+            for (int e = 0; e < 5; ++e) met[s][e] = m[e];
+        }
         __syncthreads();
-        double m2 = (threadIdx.x < ((blockDim.x + 31) >> 5)) ? sm[threadIdx.x] : 0.0;
-        m2 = warp_max(m2);
-        __syncthreads();
-        sums[0] = s3[0]; sums[1] = s3[1]; sums[2] = s3[2]; sums[3] = m2;
     }
-    double m[5];
-    sample_metric(k, a.u, a.v, a.p, a.gamma, 0, k.xCoreIn, m, sm);
-    if (threadIdx.x == 0) for (int q = 0; q < 5; ++q) met[0][q] = m[q];
-    sample_metric(k, a.u, a.v, a.p, a.gamma, 0, k.xCoreOut, m, sm);
-    if (threadIdx.x == 0) for (int q = 0; q < 5; ++q) met[1][q] = m[q];
-    sample_metric(k, a.u, a.v, a.p, a.gamma, 1, 0.0, m, sm);
-    if (threadIdx.x == 0) for (int q = 0; q < 5; ++q) met[2][q] = m[q];
-    sample_metric(k, a.u, a.v, a.p, a.gamma, 2, 0.0, m, sm);
-    if (threadIdx.x == 0) for (int q = 0; q < 5; ++q) met[3][q] = m[q];
-    __syncthreads();
     if (threadIdx.x != 0) return;
 
     const int iter = st->iter;

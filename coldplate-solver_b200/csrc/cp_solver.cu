@@ -91,7 +91,7 @@ struct cp_ctx {
     int histCap = 0;
     double* dpWin = nullptr;
     bool jacSeq = false;               // sweeps of U, then of V (jacobi_sequential)
-    int gJac = 0, gPcg = 0, gElem = 0, nbMass = 0;
+    int gJac = 0, gPcg = 0, gElem = 0, gBc = 0, nbMass = 0;
     // multigrid hierarchy (pressureSolverType 2 / 4)
     bool useMg = false;
     int mgL = 0, mgLg = 0, gMg = 0;
@@ -579,15 +579,16 @@ cudaError_t launch_coop_cfg(Kern kern, int grid, int threads, size_t smem, cudaS
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// resetBar: zero the barrier counter first (inside an iteration k_bc did)
 template <typename TC, bool Mixed>
-cp_status enqueue_momentum(cp_ctx* c, int doU, int doV, int applyBC, EvRec* rec = nullptr) {
+cp_status enqueue_momentum(cp_ctx* c, int doU, int doV, int applyBC, bool resetBar, EvRec* rec = nullptr) {
     Fields f{c->u, c->v, c->p, c->alpha, c->gamma};
     MomSys<TC> U = mom_sys<TC>(c, 0), V = mom_sys<TC>(c, 1);
     REC_BEGIN(rec, CP_K_ASSEMBLE);
     k_assemble<TC, Mixed><<<c->gElem, kThreads, 0, c->stream>>>(c->k, c->st, f, U, V, c->dE, c->dN, doU, doV);
     REC_END(rec);
     CK(cudaGetLastError());
-    CK(cudaMemsetAsync(c->barJ, 0, sizeof(unsigned), c->stream));
+    if (resetBar) CK(cudaMemsetAsync(c->barJ, 0, sizeof(unsigned), c->stream));
     JacobiOut out{c->uStar, c->vStar};
     REC_BEGIN(rec, CP_K_JACOBI);
     CK(launch_coop_cfg(c->jacSeq ? k_jacobi<TC, Mixed, true> : k_jacobi<TC, Mixed, false>, c->gJac,
@@ -599,13 +600,13 @@ cp_status enqueue_momentum(cp_ctx* c, int doU, int doV, int applyBC, EvRec* rec 
 }
 
 template <typename TV>
-cp_status enqueue_pressure(cp_ctx* c, EvRec* rec = nullptr) {
+cp_status enqueue_pressure(cp_ctx* c, bool resetBar, EvRec* rec = nullptr) {
     PcgBufs<TV> B = pcg_bufs<TV>(c);
     REC_BEGIN(rec, CP_K_MASS);
     k_mass<TV><<<c->nbMass, kThreads, 0, c->stream>>>(c->k, c->st, c->u, c->v, c->uStar, c->vStar, B.rhs, c->partM);
     REC_END(rec);
     CK(cudaGetLastError());
-    CK(cudaMemsetAsync(c->barP, 0, sizeof(unsigned), c->stream));
+    if (resetBar) CK(cudaMemsetAsync(c->barP, 0, sizeof(unsigned), c->stream));
     REC_BEGIN(rec, CP_K_PCG);
     if (c->useSa) {
         SaHier<TV> H = sa_hier<TV>(c);
@@ -626,20 +627,16 @@ cp_status enqueue_pressure(cp_ctx* c, EvRec* rec = nullptr) {
 template <typename TC, bool Mixed>
 cp_status enqueue_iteration(cp_ctx* c, EvRec* rec = nullptr) {
     REC_BEGIN(rec, CP_K_BC);
-    k_bc<<<c->gElem, kThreads, 0, c->stream>>>(c->k, c->st, c->u, c->v, c->p, c->gamma, 1);
+    k_bc<<<c->gBc, kThreads, 0, c->stream>>>(c->k, c->st, c->u, c->v, c->p, c->gamma, c->barJ, c->barP);
     REC_END(rec);
     CK(cudaGetLastError());
-    cp_status s = enqueue_momentum<TC, Mixed>(c, 1, 1, 1, rec);
+    cp_status s = enqueue_momentum<TC, Mixed>(c, 1, 1, 1, false, rec);
     if (s != CP_OK) return s;
-    s = enqueue_pressure<TC>(c, rec);
+    s = enqueue_pressure<TC>(c, false, rec);
     if (s != CP_OK) return s;
     REC_BEGIN(rec, CP_K_CORRECT);
     k_correct<<<c->gElem, kThreads, 0, c->stream>>>(c->k, c->st, c->u, c->v, c->p, c->uStar, c->vStar, c->pStar,
                                                     c->dE, c->dN);
-    REC_END(rec);
-    CK(cudaGetLastError());
-    REC_BEGIN(rec, CP_K_BC);
-    k_bc<<<c->gElem, kThreads, 0, c->stream>>>(c->k, c->st, c->u, c->v, c->p, c->gamma, 0);
     REC_END(rec);
     CK(cudaGetLastError());
     FinalizeArgs fa{c->u, c->v, c->p, c->gamma, c->partM, c->nbMass, c->hist, c->histCap, c->dpWin};
@@ -911,6 +908,7 @@ cp_status cp_create(const cp_params* prm, cp_ctx** out) {
     c->gJac = c->numSMs * (c->jacSeq ? std::min(nbJ, 3) : 1);
     c->gPcg = c->numSMs;
     c->gElem = c->numSMs * 4;
+    c->gBc = std::min(c->numSMs, (std::max(M, N) + kThreads) / kThreads);   // one boundary entry a thread
     c->nbMass = c->numSMs * 4;
     if (c->gJac > kMaxBlocks || c->gPcg > kMaxBlocks || c->nbMass > kMaxBlocks)
         return bail(fail(CP_ERR_CUDA, "too many SMs for the partial-sum buffers"));
@@ -1163,8 +1161,8 @@ static cp_status momentum_one(cp_ctx* c, int isU, double* resid, int* iters) {
     if (c->stHost->done) return fail(CP_ERR_STATE, "loop already stopped; call cp_reset_loop first");
     // reset the max-change accumulators, then assemble + solve one component
     CK(cudaMemsetAsync(&c->st->maxDU, 0, 2 * sizeof(unsigned long long), c->stream));
-    s = c->prm.precision == CP_PREC_MIXED ? enqueue_momentum<float, true>(c, isU, !isU, 0)
-                                          : enqueue_momentum<double, false>(c, isU, !isU, 0);
+    s = c->prm.precision == CP_PREC_MIXED ? enqueue_momentum<float, true>(c, isU, !isU, 0, true)
+                                          : enqueue_momentum<double, false>(c, isU, !isU, 0, true);
     if (s != CP_OK) return s;
     if ((s = read_status(c)) != CP_OK) return s;
     const unsigned long long bits = isU ? c->stHost->maxDU : c->stHost->maxDV;
@@ -1185,7 +1183,7 @@ cp_status cp_pressure(cp_ctx* c, int* iters, double* residMass) {
     if (c->stHost->done) return fail(CP_ERR_STATE, "loop already stopped; call cp_reset_loop first");
     CK(cudaMemsetAsync(c->pStar, 0, c->nElem * sizeof(double), c->stream));
     if ((s = mark_sa_stale(c)) != CP_OK) return s;
-    s = c->prm.precision == CP_PREC_MIXED ? enqueue_pressure<float>(c) : enqueue_pressure<double>(c);
+    s = c->prm.precision == CP_PREC_MIXED ? enqueue_pressure<float>(c, true) : enqueue_pressure<double>(c, true);
     if (s != CP_OK) return s;
     std::vector<double> part((size_t)4 * c->nbMass);
     CK(cudaMemcpyAsync(part.data(), c->partM, part.size() * 8, cudaMemcpyDeviceToHost, c->stream));
