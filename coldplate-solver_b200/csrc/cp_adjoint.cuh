@@ -617,9 +617,10 @@ __global__ void __launch_bounds__(1024) k_adj_g(AdjCtx a, AdjVecs V, double* Jou
 
 // r = gs g - ys y on all unknowns; partial sums of r^2 and g^2 per block
 // into part[b*2].  (gs, ys) = (1, 1): the adjoint residual; (0, -1): the
-// product y = J^T z restricted to the unknowns.
+// product y = J^T z restricted to the unknowns.  clear: y is left zero for the
+// next product.
 __global__ void k_adj_defect(KParams k, AdjVecs V, double gs, double ys, double* ru, double* rv, double* rp,
-                             double* part) {
+                             int clear, double* part) {
     __shared__ double sm[64];
     const Dims d = k.d;
     const int M = d.M, N = d.N;
@@ -629,16 +630,19 @@ __global__ void k_adj_defect(KParams k, AdjVecs V, double gs, double ys, double*
         if (t < nU) {
             const size_t c = at(d, 1 + t / (N - 2), 1 + t % (N - 2));
             const double r = gs * V.gu[c] - ys * V.yu[c];
+            if (clear) V.yu[c] = 0.0;
             ru[c] = r; acc[0] += r * r; acc[1] += V.gu[c] * V.gu[c];
         } else if (t < nU + nV) {
             const int q = t - nU;
             const size_t c = at(d, 1 + q / (N - 1), 1 + q % (N - 1));
             const double r = gs * V.gv[c] - ys * V.yv[c];
+            if (clear) V.yv[c] = 0.0;
             rv[c] = r; acc[0] += r * r; acc[1] += V.gv[c] * V.gv[c];
         } else {
             const int q = t - nU - nV;
             const size_t c = at(d, 1 + q / (N - 2), 1 + q % (N - 2));
             const double r = gs * V.gp[c] - ys * V.yp[c];
+            if (clear) V.yp[c] = 0.0;
             rp[c] = r; acc[0] += r * r; acc[1] += V.gp[c] * V.gp[c];
         }
     }
@@ -689,7 +693,8 @@ __global__ void k_adj_prec_faces(KParams k, const double* dE, const double* dN, 
 // (G^T dm)(i,j) = hy (du(i,j-1) - du(i,j)) + hx (dv(i-1,j) - dv(i,j));
 // written into the PCG rhs (TV) on the pressure unknowns.
 template <typename TV>
-__global__ void k_adj_prhs(KParams k, const double* du, const double* dv, const double* rp, TV* rhs) {
+__global__ void k_adj_prhs(KParams k, const double* du, const double* dv, const double* rp, TV* rhs, unsigned* bar) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *bar = 0u;   // the barrier counter of the solve behind it
     const Dims d = k.d;
     const int M = d.M, N = d.N, w = N - 2;
     const int n = (M - 1) * w;
@@ -839,6 +844,13 @@ __global__ void __launch_bounds__(256) k_kry_axpy(double* __restrict__ w, const 
         for (int q = 0; q < nv; ++q) a += hs[q] * B[q * L + t];
         w[t] = a;
     }
+}
+
+// dst = src / sqrt(*n2), zero for a zero norm
+__global__ void k_kry_scale_inv(double* dst, const double* src, size_t L, const double* n2) {
+    const double hn = sqrt(dmax(*n2, 0.0)), s = hn > 0.0 ? 1.0 / hn : 0.0;
+    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < L; t += (size_t)gridDim.x * blockDim.x)
+        dst[t] = s * src[t];
 }
 
 // dst = s * src

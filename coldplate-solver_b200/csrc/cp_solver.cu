@@ -140,6 +140,9 @@ struct cp_ctx {
     double* adjKry = nullptr;
     double* adjKryPart = nullptr;
     double* adjH = nullptr;
+    PoolBlock adjBlock;                // pinned: adjHost
+    double* adjHost = nullptr;         // Hessenberg entries of the last two iterations
+    cudaEvent_t adjEv[2] = {};         // their copies have landed
     int adjRestart = 30;     // m
     int adjSweeps = 6;       // equations model: transposed momentum Jacobi sweeps per preconditioner application
     int adjPIters = 6;       // multigrid-PCG iterations per preconditioner application
@@ -967,6 +970,9 @@ cp_status cp_destroy(cp_ctx* c) {
     c->mem.give_back();
     host_cache().give(c->stBlock);
     host_cache().give(c->stageBlock);
+    host_cache().give(c->adjBlock);
+    for (cudaEvent_t e : c->adjEv)
+        if (e) cudaEventDestroy(e);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -1235,13 +1241,17 @@ cp_status adjoint_alloc(cp_ctx* c) {
     if ((s = dalloc(c, &c->adjKry, (size_t)(2 * c->adjRestart + 3) * L)) != CP_OK) return s;
     if ((s = dalloc(c, &c->adjKryPart, (size_t)kKryMaxDots * kMaxBlocks)) != CP_OK) return s;
     if ((s = dalloc(c, &c->adjH, (size_t)3 * kKryMaxDots)) != CP_OK) return s;
+    static_assert(6 * kKryMaxDots * sizeof(double) <= 4096, "the pinned Hessenberg block");
+    if (!c->adjBlock.p) CK(host_cache().acquire(4096, &c->adjBlock));
+    c->adjHost = static_cast<double*>(c->adjBlock.p);
+    for (auto& e : c->adjEv)
+        if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     return CP_OK;
 }
 
 template <typename TV>
 cp_status adjoint_pcg(cp_ctx* c, const KParams& k, const double* dE, const double* dN, double* out) {
     PcgBufs<TV> B = pcg_bufs<TV>(c);
-    CK(cudaMemsetAsync(c->adjBar, 0, sizeof(unsigned), c->stream));
     if (c->useSa) {
         SaHier<TV> H = sa_hier<TV>(c);
         // the adjoint's operator is fixed over one adjoint solve: built by its
@@ -1326,7 +1336,7 @@ void kry_axpy_mdot(int nb, cudaStream_t s, double* w, const double* B, size_t L,
 template <typename TV>
 cp_status adjoint_prhs(cp_ctx* c, const KParams& k, const double* du, const double* dv, const double* rp) {
     PcgBufs<TV> B = pcg_bufs<TV>(c);
-    k_adj_prhs<TV><<<c->gElem, kThreads, 0, c->stream>>>(k, du, dv, rp, B.rhs);
+    k_adj_prhs<TV><<<c->gElem, kThreads, 0, c->stream>>>(k, du, dv, rp, B.rhs, c->adjBar);
     CK(cudaGetLastError());
     return CP_OK;
 }
@@ -1435,6 +1445,12 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
     CK(cudaMemsetAsync(kry, 0, (size_t)(2 * m + 3) * L * sizeof(double), c->stream));
     V.lu = LAM; V.lv = LAM + c->nElem; V.lc = LAM + 2 * c->nElem;
     std::vector<double> part((size_t)2 * nb);
+    // The products scatter into y with atomics, which want its lines in the L2.
+    // Where the basis vectors read in between leave them there, the kernel that
+    // reads y clears it for the next product and three launches go (253 x 127:
+    // 255 to 240 us an iteration, with the host's wait gone too); at 2048 x 1024
+    // the lines would come back from HBM one atomic at a time (1.8 to 2.1 ms).
+    const int clearY = 3 * bytes <= (size_t(4) << 20);
 
     // the reverse sweeps of both components for the adjoint vector x: the
     // adjoints of r0 and of the coefficients into UsA / VsA
@@ -1466,12 +1482,13 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
             cp_status s1 = reverse(x);
             if (s1 != CP_OK) return s1;
         }
-        for (double* y : {V.yu, V.yv, V.yp}) CK(cudaMemsetAsync(y, 0, bytes, c->stream));
+        if (!clearY)
+            for (double* y : {V.yu, V.yv, V.yp}) CK(cudaMemsetAsync(y, 0, bytes, c->stream));
         if (fixedPoint) k_adj_jt<<<nb, kThreads, 0, c->stream>>>(ac, Vx, UsA, VsA);
         else k_adj_jt_eq<<<nb, kThreads, 0, c->stream>>>(ac, Vx, nullptr, nullptr, nullptr);
         CK(cudaGetLastError());
         k_adj_defect<<<nb, kThreads, 0, c->stream>>>(k, V, gs, ys, out, out + c->nElem, out + 2 * c->nElem,
-                                                     c->adjPart);
+                                                     clearY, c->adjPart);
         CK(cudaGetLastError());
         if (rr) {
             CK(cudaMemcpyAsync(part.data(), c->adjPart, part.size() * sizeof(double), cudaMemcpyDeviceToHost,
@@ -1500,7 +1517,6 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
         cp_status s2 = c->prm.precision == CP_PREC_MIXED ? adjoint_prhs<float>(c, kp, xu, xv, rp)
                                                          : adjoint_prhs<double>(c, kp, xu, xv, rp);
         if (s2 != CP_OK) return s2;
-        CK(cudaMemsetAsync(c->adjSt, 0, sizeof(Status), c->stream));
         s2 = c->prm.precision == CP_PREC_MIXED ? adjoint_pcg<float>(c, kp, c->dE, c->dN, dc)
                                                : adjoint_pcg<double>(c, kp, c->dE, c->dN, dc);
         if (s2 != CP_OK) return s2;
@@ -1517,7 +1533,6 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
         cp_status s2 = c->prm.precision == CP_PREC_MIXED ? adjoint_prhs<float>(c, kp, V.eu, V.ev, rp)
                                                          : adjoint_prhs<double>(c, kp, V.eu, V.ev, rp);
         if (s2 != CP_OK) return s2;
-        CK(cudaMemsetAsync(c->adjSt, 0, sizeof(Status), c->stream));
         s2 = c->prm.precision == CP_PREC_MIXED ? adjoint_pcg<float>(c, kp, dEp, dNp, dc)
                                                : adjoint_pcg<double>(c, kp, dEp, dNp, dc);
         if (s2 != CP_OK) return s2;
@@ -1553,7 +1568,7 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
     double res = 1.0, gnorm = 0.0, rr = 0.0, gg = 0.0;
     int it = 0;
     bool conv = false;
-    std::vector<double> H((size_t)(m + 1) * m), gc(m), gs(m), gv(m + 1), y(m), hh(3 * kKryMaxDots);
+    std::vector<double> H((size_t)(m + 1) * m), gc(m), gs(m), gv(m + 1), y(m);
     auto Hij = [&](int i, int j) -> double& { return H[(size_t)i * m + j]; };
     // initial residual: lambda = 0, r0 = g
     if ((s = product(LAM, 1.0, 1.0, Vq(0), &rr, &gg)) != CP_OK) return s;
@@ -1569,34 +1584,19 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
         CK(cudaGetLastError());
         std::fill(gv.begin(), gv.end(), 0.0);
         gv[0] = beta;
+        // Column j's Hessenberg entries come back while iteration j + 1 runs:
+        // the device scales the next basis vector itself, and the host rotates
+        // column j (and may stop) one iteration late, so that no iteration
+        // waits for the host
         int jn = 0;
-        for (int j = 0; j < m && it < max_iter; ++j) {
-            if ((s = precondition(Vq(j), Zq(j))) != CP_OK) return s;
-            if ((s = product(Zq(j), 0.0, -1.0, W, nullptr, nullptr)) != CP_OK) return s;
-            // classical Gram-Schmidt, twice
-            double* h1 = c->adjH;
-            double* h2 = c->adjH + kKryMaxDots;
-            double* nr = c->adjH + 2 * kKryMaxDots;
-            // (each projection fused with the dot products that follow it)
-            if ((s = mdot(W, Vq(0), j + 1, h1)) != CP_OK) return s;
-            kry_axpy_mdot<false>(nb, c->stream, W, Vq(0), L, j + 1, h1, c->adjKryPart);
-            CK(cudaGetLastError());
-            k_kry_sum<<<1, 1024, 0, c->stream>>>(c->adjKryPart, nb, j + 1, h2);
-            CK(cudaGetLastError());
-            kry_axpy_mdot<true>(nb, c->stream, W, Vq(0), L, j + 1, h2, c->adjKryPart);
-            CK(cudaGetLastError());
-            k_kry_sum<<<1, 1024, 0, c->stream>>>(c->adjKryPart, nb, 1, nr);
-            CK(cudaGetLastError());
-            CK(cudaMemcpyAsync(hh.data(), c->adjH, hh.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-            CK(cudaStreamSynchronize(c->stream));
+        bool stop = false;
+        auto rotate = [&](int j) -> cp_status {
+            CK(cudaEventSynchronize(c->adjEv[j & 1]));
+            const double* hh = c->adjHost + (size_t)(j & 1) * 3 * kKryMaxDots;
             for (int i = 0; i <= j; ++i) Hij(i, j) = hh[i] + hh[kKryMaxDots + i];
             const double hn = std::sqrt(std::max(hh[2 * kKryMaxDots], 0.0));
             Hij(j + 1, j) = hn;
             if (!std::isfinite(hn)) return fail(CP_ERR_NONFINITE, "adjoint Krylov basis is not finite");
-            if (hn > 0.0) {
-                k_kry_scale<<<nb, kThreads, 0, c->stream>>>(Vq(j + 1), W, L, 1.0 / hn);
-                CK(cudaGetLastError());
-            }
             // Givens rotations of the new column; the residual estimate is |gv[j+1]|
             for (int i = 0; i < j; ++i) {
                 const double a0 = Hij(i, j), a1 = Hij(i + 1, j);
@@ -1614,8 +1614,36 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
             ++it;
             jn = j + 1;
             const double est = gnorm > 0.0 ? std::fabs(gv[j + 1]) / gnorm : 0.0;
-            if (est <= tol || hn == 0.0) break;
+            stop = est <= tol || hn == 0.0;
+            return CP_OK;
+        };
+        int launched = 0;
+        for (int j = 0; j < m && it + (j - jn) < max_iter && !stop; ++j) {
+            if ((s = precondition(Vq(j), Zq(j))) != CP_OK) return s;
+            if ((s = product(Zq(j), 0.0, -1.0, W, nullptr, nullptr)) != CP_OK) return s;
+            // classical Gram-Schmidt, twice
+            double* h1 = c->adjH;
+            double* h2 = c->adjH + kKryMaxDots;
+            double* nr = c->adjH + 2 * kKryMaxDots;
+            // (each projection fused with the dot products that follow it)
+            if ((s = mdot(W, Vq(0), j + 1, h1)) != CP_OK) return s;
+            kry_axpy_mdot<false>(nb, c->stream, W, Vq(0), L, j + 1, h1, c->adjKryPart);
+            CK(cudaGetLastError());
+            k_kry_sum<<<1, 1024, 0, c->stream>>>(c->adjKryPart, nb, j + 1, h2);
+            CK(cudaGetLastError());
+            kry_axpy_mdot<true>(nb, c->stream, W, Vq(0), L, j + 1, h2, c->adjKryPart);
+            CK(cudaGetLastError());
+            k_kry_sum<<<1, 1024, 0, c->stream>>>(c->adjKryPart, nb, 1, nr);
+            CK(cudaGetLastError());
+            CK(cudaMemcpyAsync(c->adjHost + (size_t)(j & 1) * 3 * kKryMaxDots, c->adjH, 3 * kKryMaxDots * sizeof(double),
+                               cudaMemcpyDeviceToHost, c->stream));
+            CK(cudaEventRecord(c->adjEv[j & 1], c->stream));
+            k_kry_scale_inv<<<nb, kThreads, 0, c->stream>>>(Vq(j + 1), W, L, nr);
+            CK(cudaGetLastError());
+            launched = j + 1;
+            if (j > 0 && (s = rotate(j - 1)) != CP_OK) return s;
         }
+        if (!stop && jn < launched && (s = rotate(jn)) != CP_OK) return s;
         // y = R^-1 g; lambda += Z y
         for (int i = jn - 1; i >= 0; --i) {
             double a = gv[i];
