@@ -128,4 +128,183 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg(KParams k, Status* st, c
     if (T.lead()) st->itersP = it;
 }
 
+// ------------------------------------------------------------ one cluster
+// The same solve on one cluster of 16 CTAs, for grids whose vectors fit into
+// their registers and shared memory.  A small grid's iteration on every SM is
+// two grid barriers and three trips to the L2, 7 us whatever the size; here the
+// cluster owns the grid in blocks of whole rows, K unknowns a thread with d, r,
+// z, x and A p in registers, the faces and p (with the neighbour blocks' rows
+// beside it, which they store there) in shared memory, and an iteration touches
+// no global memory at all: three cluster barriers of 0.3 us each, two of which
+// carry the sums.  What bounds it is the chain of barriers, warp sums and
+// shared-memory round trips, and 16 SMs' double-precision divisions as K grows.
+// us an iteration, here and on every SM (double): 2.9 and 6.5 at 40 x 17, 3.7
+// and 7.0 at 256 x 64, 4.5 and 7.2 at 256 x 128, 6.3 and 7.3 at 440 x 110 with
+// K = 6.  At K = 8 (512 x 128) registers spill and both take 7.4, so the line is
+// at K = 6, 49152 unknowns.
+constexpr int kClCtas = 16, kClThreads = 512, kClMaxK = 6;
+
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address that p, in this CTA's shared memory, has in CTA `rank` of the cluster
+__device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
+    unsigned a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void cluster_store(unsigned a, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_store(unsigned a, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+
+// Sums over the cluster, the same bits in every thread: each CTA stores its own
+// into all of them.  The halves of sm alternate (flip), so that a slot is
+// rewritten only after a barrier that its readers have passed too.
+struct ClusterSums {
+    double warp[2][kClThreads / 32];
+    double cta[2][2][kClCtas];
+};
+template <int NV>
+__device__ __forceinline__ void cluster_reduce(ClusterSums& sm, int& flip, double (&v)[NV]) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    flip ^= 1;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        v[k] = warp_sum(v[k]);
+        if (lane == 0) sm.warp[k][wid] = v[k];
+    }
+    __syncthreads();
+    if (wid == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const double t = warp_sum(lane < kClThreads / 32 ? sm.warp[k][lane] : 0.0);
+            if (lane < kClCtas) cluster_store(cluster_addr(&sm.cta[flip][k][blockIdx.x], lane), t);
+        }
+    }
+    cluster_barrier();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = warp_sum(lane < kClCtas ? sm.cta[flip][k][lane] : 0.0);
+}
+
+// Rows a CTA owns, unknowns a thread (0: too large), and bytes of shared memory: p on R + 2
+// rows, the north faces on R + 1 and the east faces on R, each w + 2 wide.
+inline __host__ __device__ int pcg_cl_rows(int M) { return (M - 1 + kClCtas - 1) / kClCtas; }
+inline int pcg_cl_k(int M, int N) {
+    const long cells = (long)pcg_cl_rows(M) * (N - 2);
+    for (int K : {1, 2, 4, kClMaxK})
+        if (cells <= (long)K * kClThreads) return K;
+    return 0;
+}
+inline size_t pcg_cl_smem(int M, int N, size_t es) { return (size_t)(3 * pcg_cl_rows(M) + 3) * N * es; }
+// its largest value: one row a CTA (or rows of two unknowns) of 6 x 512 unknowns in double
+constexpr size_t kClSmemMax = 6 * (kClMaxK * kClThreads + 2) * 8;
+
+template <typename TV, int K>
+__global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(KParams k, Status* st, const double* dE, const double* dN,
+                                                               const TV* rhs, double* pStar) {
+    if (st->done) return;
+    extern __shared__ __align__(128) double dsm[];
+    __shared__ ClusterSums sm;
+    const Dims d = k.d;
+    const int M = d.M, N = d.N, w = N - 2, W = N;
+    const int rank = blockIdx.x, tid = threadIdx.x;
+    const int R = pcg_cl_rows(M), i0 = 1 + rank * R, rows = max(0, min(R, M - i0));
+    TV* const sp = reinterpret_cast<TV*>(dsm);    // row l of the block at (l + 1) W, column j at j
+    TV* const sn = sp + (R + 2) * W;              // likewise; row -1 is the block below's
+    TV* const se = sn + (R + 1) * W;              // row l at l W
+    for (int t = tid; t < (3 * R + 3) * W; t += kClThreads) sp[t] = (TV)0;
+    __syncthreads();
+    TV dd[K], r[K], z[K], x[K], ap[K];
+    int at0[K];     // place in sp, 0 past the block's unknowns
+    double acc[2] = {0.0, 0.0};
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+        const int q = tid + m * kClThreads, l = q / w, j = 1 + q - l * w, i = i0 + l;
+        dd[m] = (TV)1;
+        r[m] = z[m] = x[m] = ap[m] = (TV)0;
+        at0[m] = 0;
+        if (l >= rows) continue;
+        const size_t c = at(d, i, j);
+        const double aE = k.rho * dE[c] * k.hy;
+        const double aW = (j > 1) ? k.rho * dE[c - 1] * k.hy : 0.0;
+        const double aN = (i < M - 1) ? k.rho * dN[c] * k.hx : 0.0;
+        const double aS = (i > 1) ? k.rho * dN[c - d.P] * k.hx : 0.0;
+        double aP = aE + aW + aN + aS;
+        if (aP < 1e-20) aP = 1.0;
+        at0[m] = (l + 1) * W + j;
+        se[l * W + j] = j < w ? (TV)aE : (TV)0;
+        sn[at0[m]] = (TV)aN;
+        if (l == 0) sn[j] = (TV)aS;
+        dd[m] = (TV)aP;
+        r[m] = rhs[c];
+        z[m] = r[m] / dd[m];
+        acc[1] += (double)r[m] * (double)z[m];
+    }
+    // the neighbour blocks' rows beside this block's: north of rank - 1, south of rank + 1
+    const bool hasS = rank > 0 && rows > 0, hasN = rows > 0 && i0 + rows <= M - 1;
+    const unsigned toS = cluster_addr(sp + (R + 1) * W, hasS ? rank - 1 : rank),
+                   toN = cluster_addr(sp, hasN ? rank + 1 : rank);
+    int flip = 0;
+    cluster_barrier();   // every block's shared memory is there, and cleared
+    cluster_reduce(sm, flip, acc);
+    double rz = acc[1];
+    TV bt = (TV)0;
+    int it = 0;
+    for (; it < k.maxP; ++it) {
+#pragma unroll
+        for (int m = 0; m < K; ++m) {
+            const int o = at0[m];
+            if (!o) continue;
+            const TV p = it ? (TV)(z[m] + bt * sp[o]) : z[m];
+            sp[o] = p;
+            if (hasS && o < 2 * W) cluster_store(toS + (unsigned)((o - W) * sizeof(TV)), p);
+            if (hasN && o >= rows * W) cluster_store(toN + (unsigned)((o - rows * W) * sizeof(TV)), p);
+        }
+        cluster_barrier();
+        double v[1] = {0.0};
+#pragma unroll
+        for (int m = 0; m < K; ++m) {
+            const int o = at0[m];
+            if (!o) continue;
+            const TV pc = sp[o];
+            const TV a = dd[m] * pc - se[o - W] * sp[o + 1] - se[o - W - 1] * sp[o - 1] - sn[o] * sp[o + W] -
+                         sn[o - W] * sp[o - W];
+            ap[m] = a;
+            v[0] += (double)pc * (double)a;
+        }
+        cluster_reduce(sm, flip, v);
+        if (fabs(v[0]) < 1e-20) break;
+        const TV al = (TV)(rz / v[0]);
+        acc[0] = acc[1] = 0.0;
+#pragma unroll
+        for (int m = 0; m < K; ++m) {
+            const int o = at0[m];
+            if (!o) continue;
+            x[m] = x[m] + al * sp[o];
+            r[m] = r[m] - al * ap[m];
+            z[m] = r[m] / dd[m];
+            acc[0] += (double)r[m] * (double)r[m];
+            acc[1] += (double)r[m] * (double)z[m];
+        }
+        cluster_reduce(sm, flip, acc);
+        if (sqrt(acc[0]) < k.pTol) break;
+        bt = (TV)(acc[1] / rz);
+        rz = acc[1];
+    }
+    // p'(:, N-1) = 0 (pressure_solver.cpp:814)
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+        const int q = tid + m * kClThreads, l = q / w, j = 1 + q - l * w;
+        if (!at0[m]) continue;
+        const size_t c = at(d, i0 + l, j);
+        pStar[c] = (double)x[m];
+        if (j == w) pStar[c + 1] = 0.0;
+    }
+    if (rank == 0 && tid == 0) st->itersP = it;
+}
+
 }  // namespace cp

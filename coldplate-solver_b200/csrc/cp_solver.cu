@@ -92,6 +92,7 @@ struct cp_ctx {
     double* dpWin = nullptr;
     bool jacSeq = false;               // sweeps of U, then of V (jacobi_sequential)
     int gJac = 0, gPcg = 0, gElem = 0, gBc = 0, nbMass = 0;
+    int clK = 0;                       // Jacobi-PCG on one cluster: unknowns a thread (0: on every SM)
     // multigrid hierarchy (pressureSolverType 2 / 4)
     bool useMg = false;
     int mgL = 0, mgLg = 0, gMg = 0;
@@ -582,6 +583,57 @@ cudaError_t launch_coop_cfg(Kern kern, int grid, int threads, size_t smem, cudaS
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// The Jacobi-PCG on one cluster (k_pcg_cluster) with K unknowns a thread
+template <typename TV>
+using PcgClusterFn = void (*)(KParams, Status*, const double*, const double*, const TV*, double*);
+template <typename TV>
+PcgClusterFn<TV> pcg_cluster_fn(int K) {
+    return K == 1 ? k_pcg_cluster<TV, 1> : K == 2 ? k_pcg_cluster<TV, 2> : K == 4 ? k_pcg_cluster<TV, 4>
+                                                                         : k_pcg_cluster<TV, kClMaxK>;
+}
+
+cudaLaunchConfig_t pcg_cluster_config(const Dims& d, size_t es, cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kClCtas);
+    cfg.blockDim = dim3(kClThreads);
+    cfg.dynamicSmemBytes = pcg_cl_smem(d.M, d.N, es);
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = kClCtas;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Unknowns a thread of the cluster's PCG on this grid; 0 where the grid is too
+// large for it or the device cannot place the cluster.
+template <typename TV>
+int pcg_cluster_k(const Dims& d) {
+    const int K = pcg_cl_k(d.M, d.N);
+    if (K == 0) return 0;
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = pcg_cluster_config(d, sizeof(TV), &attr);
+    int n = 0;
+    const PcgClusterFn<TV> f = pcg_cluster_fn<TV>(K);
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmemMax) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess && n >= 1)
+        return K;
+    (void)cudaGetLastError();
+    return 0;
+}
+
+template <typename TV>
+cudaError_t launch_pcg(const cp_ctx* c, const KParams& k, Status* st, const double* dE, const double* dN,
+                       const PcgBufs<TV>& B, double* out, double* part, unsigned* bar) {
+    if (c->clK == 0) return launch_coop_cfg(k_pcg<TV>, c->gPcg, kPcgThreads, 0, c->stream, k, st, dE, dN, B, out, part, bar);
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg = pcg_cluster_config(k.d, sizeof(TV), &attr);
+    cfg.stream = c->stream;
+    return cudaLaunchKernelEx(&cfg, pcg_cluster_fn<TV>(c->clK), k, st, dE, dN, (const TV*)B.rhs, out);
+}
+
 // resetBar: zero the barrier counter first (inside an iteration k_bc did)
 template <typename TC, bool Mixed>
 cp_status enqueue_momentum(cp_ctx* c, int doU, int doV, int applyBC, bool resetBar, EvRec* rec = nullptr) {
@@ -620,8 +672,7 @@ cp_status enqueue_pressure(cp_ctx* c, bool resetBar, EvRec* rec = nullptr) {
         CK(launch_coop_cfg(k_pcg_mg<TV>, c->gMg, kMgThreads, kMgDynSmem, c->stream, c->k, c->st,
                            (const double*)c->dE, (const double*)c->dN, B, H, c->pStar, c->partP, c->barP, c->mgMaps));
     } else {
-        CK(launch_coop_cfg(k_pcg<TV>, c->gPcg, kPcgThreads, 0, c->stream, c->k, c->st, (const double*)c->dE, (const double*)c->dN, B,
-                       c->pStar, c->partP, c->barP));
+        CK(launch_pcg<TV>(c, c->k, c->st, c->dE, c->dN, B, c->pStar, c->partP, c->barP));
     }
     REC_END(rec);
     return CP_OK;
@@ -922,6 +973,7 @@ cp_status cp_create(const cp_params* prm, cp_ctx** out) {
     const char* cyc = getenv("CP_PRESSURE_CYCLE");
     c->useSa = prm->pressureSolverType == 4 && !(cyc && strcmp(cyc, "pairs") == 0);
     if (c->useSa && (s = sa_build(c)) != CP_OK) return bail(s);
+    if (!c->useMg) c->clK = c->prm.precision == CP_PREC_MIXED ? pcg_cluster_k<float>(c->d) : pcg_cluster_k<double>(c->d);
     if ((s = dalloc(c, &c->partJ, (size_t)4 * c->gJac)) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->partM, (size_t)4 * c->nbMass)) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->partP, (size_t)4 * std::max(c->gPcg, c->gMg))) != CP_OK) return bail(s);
@@ -1266,7 +1318,7 @@ cp_status adjoint_pcg(cp_ctx* c, const KParams& k, const double* dE, const doubl
         CK(launch_coop_cfg(k_pcg_mg<TV>, c->gMg, kMgThreads, kMgDynSmem, c->stream, k, c->adjSt, dE, dN, B, H, out,
                            c->adjPart, c->adjBar, c->mgMaps));
     } else {
-        CK(launch_coop_cfg(k_pcg<TV>, c->gPcg, kPcgThreads, 0, c->stream, k, c->adjSt, dE, dN, B, out, c->adjPart, c->adjBar));
+        CK(launch_pcg<TV>(c, k, c->adjSt, dE, dN, B, out, c->adjPart, c->adjBar));
     }
     return CP_OK;
 }
@@ -1729,7 +1781,8 @@ extern "C" cp_status cp_adjoint_probe(cp_ctx* c, int op, const double* x, double
 
 // ======================================================================== no-allocation entry point
 // cp_pressure_noalloc: the Jacobi-PCG pressure-correction solve (k_mass +
-// k_pcg<double>, the kernels behind cp_pressure for pressureSolverType 1)
+// k_pcg<double>, the kernels behind cp_pressure for pressureSolverType 1 on
+// grids too large for one cluster, on any row pitch)
 // for callers that cannot allocate device memory.  All of its working
 // memory lives in one file-scope device array of fixed size, below; the
 // caller provides only the inputs and the output.
