@@ -578,6 +578,132 @@ __global__ void __launch_bounds__(Seq ? kJacSegThreads : kJacThreads, Seq ? 3 : 
     }
 }
 
+// The same on two clusters, one a component, for grids small enough
+// (cluster_unknowns of both): the six coefficients of a thread's unknowns stay
+// in registers and the iterate, with the neighbour blocks' rows beside a
+// block's, in two buffers of shared memory, so that a sweep is one pass over
+// them and one cluster barrier, which carries the sum too.  Per unknown the
+// arithmetic is jacobi_run's, so u* and v* are the same bits.  us for the
+// sweeps, here and on every SM: 15.6 and 34.0 at 40 x 17 (11.5 sweeps, double),
+// 27.2 and 56.6 at 256 x 64 (19.5), 38.6 and 75.0 at 253 x 127 (26.6), 40.7 and
+// 60.1 at 400 x 100 (float, 19.4), 47.6 and 61.0 there in double with K = 6.
+constexpr size_t kJacClSmemMax = 2 * 3 * (kClMaxK * kClThreads + 3) * 8;   // one row a CTA, or rows of two unknowns
+inline size_t jac_cl_smem(const Dims& d, size_t es) { return (size_t)2 * (cluster_rows(d.M - 1) + 2) * (d.N + 1) * es; }
+inline int jac_cl_k(const Dims& d) {
+    const int U = cluster_unknowns(d.M - 1, d.N - 2), V = cluster_unknowns(d.M - 2, d.N - 1);
+    return U && V ? (U > V ? U : V) : 0;
+}
+
+template <typename TC, bool Mixed, bool IsU, int K>
+__device__ __forceinline__ void jacobi_cluster(const KParams& k, Status* st, const MomSys<TC>& S, const double* field,
+                                               double* out, double maxVel, bool outlet, TC* buf, ClusterSums& sm) {
+    const Dims d = k.d;
+    int i1, j1;
+    mom_range<IsU>(d, i1, j1);
+    const int rank = blockIdx.x % kClCtas, tid = threadIdx.x, W = d.N + 1;
+    const int R = cluster_rows(i1), i0 = 1 + rank * R, rows = max(0, min(R, i1 + 1 - i0));
+    const int len = (R + 2) * W;    // a buffer: row l of the block at (l + 1) W, column j at j
+    for (int t = tid; t < 2 * len; t += kClThreads) buf[t] = (TC)0;
+    __syncthreads();
+    TC aP[K], aE[K], aW[K], aN[K], aS[K], b[K];
+    int at0[K];     // place in a buffer, 0 past the block's unknowns
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+        const int q = tid + m * kClThreads, l = q / j1, j = 1 + q - l * j1;
+        at0[m] = 0;
+        aP[m] = aE[m] = aW[m] = aN[m] = aS[m] = b[m] = (TC)0;
+        if (l >= rows) continue;
+        const size_t c = at(d, i0 + l, j);
+        at0[m] = (l + 1) * W + j;
+        aP[m] = S.aP[c];
+        aE[m] = S.aE[c];
+        aW[m] = S.aW[c];
+        aN[m] = S.aN[c];
+        aS[m] = S.aS[c];
+        b[m] = S.b[c];
+        // the current field, or zero in the mixed form
+        if constexpr (!Mixed) {
+            buf[at0[m]] = field[c];
+            if (l == 0 && rank > 0) buf[j] = field[c - d.P];
+            if (l == rows - 1 && i0 + l < i1) buf[at0[m] + W] = field[c + d.P];
+        }
+    }
+    // the neighbour blocks' rows beside this block's: north of rank - 1, south of rank + 1
+    const bool hasS = rank > 0 && rows > 0, hasN = rows > 0 && i0 + rows <= i1;
+    const unsigned toS = cluster_addr(buf + (R + 1) * W, hasS ? rank - 1 : rank),
+                   toN = cluster_addr(buf, hasN ? rank + 1 : rank);
+    const double lim = k.momTol * k.momTol * (double)(IsU ? k.nU : k.nV);
+    int flip = 0, its = 0;
+    bool on = k.maxMom > 0;
+    const TC* x = buf;
+    cluster_barrier();   // every block's shared memory is there, and loaded
+    while (on) {
+        const int nx = its & 1 ? 0 : len;
+        TC* const xn = buf + nx;
+        double acc[1] = {0.0};
+#pragma unroll
+        for (int m = 0; m < K; ++m) {
+            const int o = at0[m];
+            if (!o) continue;
+            const TC xP = x[o];
+            // S, W, P, E, N order of the reference's CSR rows
+            TC Ax = (TC)0;
+            Ax += (-aS[m]) * x[o - W];
+            Ax += (-aW[m]) * x[o - 1];
+            Ax += aP[m] * xP;
+            Ax += (-aE[m]) * x[o + 1];
+            Ax += (-aN[m]) * x[o + W];
+            const TC r = b[m] - Ax;
+            const TC y = (TC)(xP + r / aP[m]);
+            acc[0] += (double)r * (double)r;
+            xn[o] = y;
+            if (hasS && o < 2 * W) cluster_store(toS + (unsigned)((nx + o - W) * sizeof(TC)), y);
+            if (hasN && o >= rows * W) cluster_store(toN + (unsigned)((nx + o - rows * W) * sizeof(TC)), y);
+        }
+        cluster_reduce(sm, flip, rank, acc);
+        x = xn;
+        on = ++its < k.maxMom && !(acc[0] < lim);
+    }
+    double mx = 0.0;
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+        const int q = tid + m * kClThreads, l = q / j1, j = 1 + q - l * j1;
+        if (!at0[m]) continue;
+        const size_t c = at(d, i0 + l, j);
+        double xv = (double)x[at0[m]];
+        if (Mixed) xv += field[c];
+        const double nv = dclamp(xv, -maxVel, maxVel);
+        mx = dmax(mx, fabs(nv - field[c]));
+        out[c] = nv;
+        if (outlet && j == j1) out[c + 1] = nv;
+    }
+    mx = warp_max(mx);
+    if ((tid & 31) == 0) atomic_max_nonneg(IsU ? &st->maxDU : &st->maxDV, mx);
+    if (rank == 0 && tid == 0) {
+        if (IsU) st->itersU = its;
+        else st->itersV = its;
+    }
+}
+
+template <typename TC, bool Mixed, int K>
+__global__ void __launch_bounds__(kClThreads, 1) k_jacobi_cluster(KParams k, Status* st, MomSys<TC> U, MomSys<TC> V,
+                                                                  const double* u, const double* v, JacobiOut out,
+                                                                  const double* gamma, int doU, int doV, int applyBC) {
+    if (st->done) return;
+    extern __shared__ __align__(128) double jsm[];
+    __shared__ ClusterSums sm;
+    const int iter = st->iter;
+    const double maxVel = max_vel(inlet_velocity(k, iter));
+    TC* const buf = reinterpret_cast<TC*>(jsm);
+    if (blockIdx.x < kClCtas) {
+        if (doU) jacobi_cluster<TC, Mixed, true, K>(k, st, U, u, out.uStar, maxVel, applyBC, buf, sm);
+    } else {
+        if (doV) jacobi_cluster<TC, Mixed, false, K>(k, st, V, v, out.vStar, maxVel, applyBC, buf, sm);
+    }
+    if (applyBC)
+        apply_bc_const(k, iter, out.uStar, out.vStar, gamma, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
 // ------------------------------------------------------------------ mass
 // One pass over cells (i, j) in [1, M-1] x [1, N-1]: RMS sums of u* - u and
 // v* - v over their unknowns (iterations.cpp:507-525), the mass imbalance

@@ -142,64 +142,9 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg(KParams k, Status* st, c
 // and 7.0 at 256 x 64, 4.5 and 7.2 at 256 x 128, 6.3 and 7.3 at 440 x 110 with
 // K = 6.  At K = 8 (512 x 128) registers spill and both take 7.4, so the line is
 // at K = 6, 49152 unknowns.
-constexpr int kClCtas = 16, kClThreads = 512, kClMaxK = 6;
-
-__device__ __forceinline__ void cluster_barrier() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// The address that p, in this CTA's shared memory, has in CTA `rank` of the cluster
-__device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
-    unsigned a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
-    return a;
-}
-__device__ __forceinline__ void cluster_store(unsigned a, double v) {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-__device__ __forceinline__ void cluster_store(unsigned a, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-
-// Sums over the cluster, the same bits in every thread: each CTA stores its own
-// into all of them.  The halves of sm alternate (flip), so that a slot is
-// rewritten only after a barrier that its readers have passed too.
-struct ClusterSums {
-    double warp[2][kClThreads / 32];
-    double cta[2][2][kClCtas];
-};
-template <int NV>
-__device__ __forceinline__ void cluster_reduce(ClusterSums& sm, int& flip, double (&v)[NV]) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    flip ^= 1;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        v[k] = warp_sum(v[k]);
-        if (lane == 0) sm.warp[k][wid] = v[k];
-    }
-    __syncthreads();
-    if (wid == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            const double t = warp_sum(lane < kClThreads / 32 ? sm.warp[k][lane] : 0.0);
-            if (lane < kClCtas) cluster_store(cluster_addr(&sm.cta[flip][k][blockIdx.x], lane), t);
-        }
-    }
-    cluster_barrier();
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = warp_sum(lane < kClCtas ? sm.cta[flip][k][lane] : 0.0);
-}
-
-// Rows a CTA owns, unknowns a thread (0: too large), and bytes of shared memory: p on R + 2
-// rows, the north faces on R + 1 and the east faces on R, each w + 2 wide.
-inline __host__ __device__ int pcg_cl_rows(int M) { return (M - 1 + kClCtas - 1) / kClCtas; }
-inline int pcg_cl_k(int M, int N) {
-    const long cells = (long)pcg_cl_rows(M) * (N - 2);
-    for (int K : {1, 2, 4, kClMaxK})
-        if (cells <= (long)K * kClThreads) return K;
-    return 0;
-}
-inline size_t pcg_cl_smem(int M, int N, size_t es) { return (size_t)(3 * pcg_cl_rows(M) + 3) * N * es; }
+// Bytes of shared memory: p on R + 2 rows, the north faces on R + 1 and the
+// east faces on R, each w + 2 wide.
+inline size_t pcg_cl_smem(int M, int N, size_t es) { return (size_t)(3 * cluster_rows(M - 1) + 3) * N * es; }
 // its largest value: one row a CTA (or rows of two unknowns) of 6 x 512 unknowns in double
 constexpr size_t kClSmemMax = 6 * (kClMaxK * kClThreads + 2) * 8;
 
@@ -212,7 +157,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(KParams k, Status
     const Dims d = k.d;
     const int M = d.M, N = d.N, w = N - 2, W = N;
     const int rank = blockIdx.x, tid = threadIdx.x;
-    const int R = pcg_cl_rows(M), i0 = 1 + rank * R, rows = max(0, min(R, M - i0));
+    const int R = cluster_rows(M - 1), i0 = 1 + rank * R, rows = max(0, min(R, M - i0));
     TV* const sp = reinterpret_cast<TV*>(dsm);    // row l of the block at (l + 1) W, column j at j
     TV* const sn = sp + (R + 2) * W;              // likewise; row -1 is the block below's
     TV* const se = sn + (R + 1) * W;              // row l at l W
@@ -250,7 +195,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(KParams k, Status
                    toN = cluster_addr(sp, hasN ? rank + 1 : rank);
     int flip = 0;
     cluster_barrier();   // every block's shared memory is there, and cleared
-    cluster_reduce(sm, flip, acc);
+    cluster_reduce(sm, flip, rank, acc);
     double rz = acc[1];
     TV bt = (TV)0;
     int it = 0;
@@ -276,7 +221,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(KParams k, Status
             ap[m] = a;
             v[0] += (double)pc * (double)a;
         }
-        cluster_reduce(sm, flip, v);
+        cluster_reduce(sm, flip, rank, v);
         if (fabs(v[0]) < 1e-20) break;
         const TV al = (TV)(rz / v[0]);
         acc[0] = acc[1] = 0.0;
@@ -290,7 +235,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(KParams k, Status
             acc[0] += (double)r[m] * (double)r[m];
             acc[1] += (double)r[m] * (double)z[m];
         }
-        cluster_reduce(sm, flip, acc);
+        cluster_reduce(sm, flip, rank, acc);
         if (sqrt(acc[0]) < k.pTol) break;
         bt = (TV)(acc[1] / rz);
         rz = acc[1];

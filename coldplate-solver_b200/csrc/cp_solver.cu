@@ -92,7 +92,7 @@ struct cp_ctx {
     double* dpWin = nullptr;
     bool jacSeq = false;               // sweeps of U, then of V (jacobi_sequential)
     int gJac = 0, gPcg = 0, gElem = 0, gBc = 0, nbMass = 0;
-    int clK = 0;                       // Jacobi-PCG on one cluster: unknowns a thread (0: on every SM)
+    int clK = 0, clJacK = 0;           // Jacobi-PCG / sweeps on clusters: unknowns a thread (0: on every SM)
     // multigrid hierarchy (pressureSolverType 2 / 4)
     bool useMg = false;
     int mgL = 0, mgLg = 0, gMg = 0;
@@ -583,20 +583,13 @@ cudaError_t launch_coop_cfg(Kern kern, int grid, int threads, size_t smem, cudaS
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-// The Jacobi-PCG on one cluster (k_pcg_cluster) with K unknowns a thread
-template <typename TV>
-using PcgClusterFn = void (*)(KParams, Status*, const double*, const double*, const TV*, double*);
-template <typename TV>
-PcgClusterFn<TV> pcg_cluster_fn(int K) {
-    return K == 1 ? k_pcg_cluster<TV, 1> : K == 2 ? k_pcg_cluster<TV, 2> : K == 4 ? k_pcg_cluster<TV, 4>
-                                                                         : k_pcg_cluster<TV, kClMaxK>;
-}
-
-cudaLaunchConfig_t pcg_cluster_config(const Dims& d, size_t es, cudaLaunchAttribute* attr) {
+// ---- kernels that run on clusters of kClCtas CTAs (small grids)
+cudaLaunchConfig_t cluster_config(int clusters, size_t smem, cudaStream_t s, cudaLaunchAttribute* attr) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kClCtas);
+    cfg.gridDim = dim3(clusters * kClCtas);
     cfg.blockDim = dim3(kClThreads);
-    cfg.dynamicSmemBytes = pcg_cl_smem(d.M, d.N, es);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
     attr->id = cudaLaunchAttributeClusterDimension;
     attr->val.clusterDim.x = kClCtas;
     attr->val.clusterDim.y = 1;
@@ -606,22 +599,50 @@ cudaLaunchConfig_t pcg_cluster_config(const Dims& d, size_t es, cudaLaunchAttrib
     return cfg;
 }
 
-// Unknowns a thread of the cluster's PCG on this grid; 0 where the grid is too
-// large for it or the device cannot place the cluster.
+// Whether the device can place a cluster of the kernel
+template <typename Kern>
+bool cluster_fits(Kern f, size_t smem, size_t smemMax) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_config(1, smem, nullptr, &attr);
+    int n = 0;
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemMax) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess && n >= 1)
+        return true;
+    (void)cudaGetLastError();
+    return false;
+}
+
+// The Jacobi-PCG (k_pcg_cluster) and the sweeps (k_jacobi_cluster) with K
+// unknowns a thread
+template <typename TV>
+using PcgClusterFn = void (*)(KParams, Status*, const double*, const double*, const TV*, double*);
+template <typename TV>
+PcgClusterFn<TV> pcg_cluster_fn(int K) {
+    return K == 1 ? k_pcg_cluster<TV, 1> : K == 2 ? k_pcg_cluster<TV, 2> : K == 4 ? k_pcg_cluster<TV, 4>
+                                                                         : k_pcg_cluster<TV, kClMaxK>;
+}
+template <typename TC>
+using JacClusterFn = void (*)(KParams, Status*, MomSys<TC>, MomSys<TC>, const double*, const double*, JacobiOut,
+                              const double*, int, int, int);
+template <typename TC, bool Mixed>
+JacClusterFn<TC> jac_cluster_fn(int K) {
+    return K == 1 ? k_jacobi_cluster<TC, Mixed, 1> : K == 2 ? k_jacobi_cluster<TC, Mixed, 2>
+                                               : K == 4 ? k_jacobi_cluster<TC, Mixed, 4>
+                                                        : k_jacobi_cluster<TC, Mixed, kClMaxK>;
+}
+
+// Unknowns a thread of each on this grid; 0 where the grid is too large or the
+// device cannot place the cluster
 template <typename TV>
 int pcg_cluster_k(const Dims& d) {
-    const int K = pcg_cl_k(d.M, d.N);
-    if (K == 0) return 0;
-    cudaLaunchAttribute attr;
-    const cudaLaunchConfig_t cfg = pcg_cluster_config(d, sizeof(TV), &attr);
-    int n = 0;
-    const PcgClusterFn<TV> f = pcg_cluster_fn<TV>(K);
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmemMax) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&n, f, &cfg) == cudaSuccess && n >= 1)
-        return K;
-    (void)cudaGetLastError();
-    return 0;
+    const int K = cluster_unknowns(d.M - 1, d.N - 2);
+    return K && cluster_fits(pcg_cluster_fn<TV>(K), pcg_cl_smem(d.M, d.N, sizeof(TV)), kClSmemMax) ? K : 0;
+}
+template <typename TC, bool Mixed>
+int jac_cluster_k(const Dims& d) {
+    const int K = jac_cl_k(d);
+    return K && cluster_fits(jac_cluster_fn<TC, Mixed>(K), jac_cl_smem(d, sizeof(TC)), kJacClSmemMax) ? K : 0;
 }
 
 template <typename TV>
@@ -629,9 +650,22 @@ cudaError_t launch_pcg(const cp_ctx* c, const KParams& k, Status* st, const doub
                        const PcgBufs<TV>& B, double* out, double* part, unsigned* bar) {
     if (c->clK == 0) return launch_coop_cfg(k_pcg<TV>, c->gPcg, kPcgThreads, 0, c->stream, k, st, dE, dN, B, out, part, bar);
     cudaLaunchAttribute attr;
-    cudaLaunchConfig_t cfg = pcg_cluster_config(k.d, sizeof(TV), &attr);
-    cfg.stream = c->stream;
+    const cudaLaunchConfig_t cfg = cluster_config(1, pcg_cl_smem(k.d.M, k.d.N, sizeof(TV)), c->stream, &attr);
     return cudaLaunchKernelEx(&cfg, pcg_cluster_fn<TV>(c->clK), k, st, dE, dN, (const TV*)B.rhs, out);
+}
+
+template <typename TC, bool Mixed>
+cudaError_t launch_jacobi(const cp_ctx* c, const MomSys<TC>& U, const MomSys<TC>& V, int doU, int doV, int applyBC) {
+    const JacobiOut out{c->uStar, c->vStar};
+    if (c->clJacK == 0)
+        return launch_coop_cfg(c->jacSeq ? k_jacobi<TC, Mixed, true> : k_jacobi<TC, Mixed, false>, c->gJac,
+                               c->jacSeq ? kJacSegThreads : kJacThreads, 0, c->stream, c->k, c->st, U, V,
+                               (const double*)c->u, (const double*)c->v, (TC*)c->xb[0], (TC*)c->xb[1], (TC*)c->xb[2],
+                               (TC*)c->xb[3], out, (const double*)c->gamma, c->partJ, c->barJ, doU, doV, applyBC);
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg = cluster_config(2, jac_cl_smem(c->d, sizeof(TC)), c->stream, &attr);
+    return cudaLaunchKernelEx(&cfg, jac_cluster_fn<TC, Mixed>(c->clJacK), c->k, c->st, U, V, (const double*)c->u,
+                              (const double*)c->v, out, (const double*)c->gamma, doU, doV, applyBC);
 }
 
 // resetBar: zero the barrier counter first (inside an iteration k_bc did)
@@ -644,12 +678,8 @@ cp_status enqueue_momentum(cp_ctx* c, int doU, int doV, int applyBC, bool resetB
     REC_END(rec);
     CK(cudaGetLastError());
     if (resetBar) CK(cudaMemsetAsync(c->barJ, 0, sizeof(unsigned), c->stream));
-    JacobiOut out{c->uStar, c->vStar};
     REC_BEGIN(rec, CP_K_JACOBI);
-    CK(launch_coop_cfg(c->jacSeq ? k_jacobi<TC, Mixed, true> : k_jacobi<TC, Mixed, false>, c->gJac,
-                   c->jacSeq ? kJacSegThreads : kJacThreads, 0, c->stream, c->k, c->st, U, V, (const double*)c->u,
-                   (const double*)c->v, (TC*)c->xb[0], (TC*)c->xb[1], (TC*)c->xb[2], (TC*)c->xb[3], out,
-                   (const double*)c->gamma, c->partJ, c->barJ, doU, doV, applyBC));
+    CK((launch_jacobi<TC, Mixed>(c, U, V, doU, doV, applyBC)));
     REC_END(rec);
     return CP_OK;
 }
@@ -973,6 +1003,7 @@ cp_status cp_create(const cp_params* prm, cp_ctx** out) {
     const char* cyc = getenv("CP_PRESSURE_CYCLE");
     c->useSa = prm->pressureSolverType == 4 && !(cyc && strcmp(cyc, "pairs") == 0);
     if (c->useSa && (s = sa_build(c)) != CP_OK) return bail(s);
+    c->clJacK = c->prm.precision == CP_PREC_MIXED ? jac_cluster_k<float, true>(c->d) : jac_cluster_k<double, false>(c->d);
     if (!c->useMg) c->clK = c->prm.precision == CP_PREC_MIXED ? pcg_cluster_k<float>(c->d) : pcg_cluster_k<double>(c->d);
     if ((s = dalloc(c, &c->partJ, (size_t)4 * c->gJac)) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->partM, (size_t)4 * c->nbMass)) != CP_OK) return bail(s);
