@@ -58,12 +58,12 @@ ADJ_FD_NOTE = ("not checked at this state; vs central FD (h 1e-4) at converged s
 # ncu captures of the dominant kernels (profiles/): DRAM bytes read + written
 PCG_MG_CAPTURE_BYTES = (762.0 + 1447.7) * 1e6     # k_pcg_mg<float>, one launch (32 x 64 tiles)
 PCG_MG_CAPTURE_ITERS = 30
-# k_pcg_sa<float>: four consecutive launches (outer iterations 20-23 of the
-# mixed solve, one of them rebuilding the coarse operators), 58 CG iterations
-PCG_SA_CAPTURE_BYTES = (6459.0 + 3920.0) * 1e6
-PCG_SA_CAPTURE_ITERS = 58
-THERMAL_CAPTURE_BYTES_PER_CELL_ITER = 693.0        # k_th_bicgstab<false, double>, 512 x 256 x 12 (78 iterations)
-THERMAL_MIXED_CAPTURE_BYTES_PER_CELL_ITER = 406.0  # k_th_bicgstab<false, float>, the same case (85 iterations)
+# k_pcg_sa<float>: three consecutive launches (outer iterations 20-22 of the
+# mixed solve, one of them rebuilding the coarse operators), 43 CG iterations
+PCG_SA_CAPTURE_BYTES = (2200.4 + 2027.4) * 1e6
+PCG_SA_CAPTURE_ITERS = 43
+THERMAL_CAPTURE_BYTES_PER_CELL_ITER = 689.0        # k_th_bicgstab<false, double>, 512 x 256 x 12 (78 iterations)
+THERMAL_MIXED_CAPTURE_BYTES_PER_CELL_ITER = 415.0  # k_th_bicgstab<false, float>, the same case (90 iterations)
 
 
 def parse():
@@ -582,12 +582,13 @@ def thermal_leg(Simple, torch, args) -> dict:
     its_f = max(r["iterations"] for r in fwd)
     its_a = max(r["iterations"] for r in adj)
     # algorithmic bytes per cell and BiCGStab iteration, FP64 words, every
-    # vector and coefficient once per phase that needs it: level 0 85.5 (the
-    # two vector updates fused with pre-smoothing, 8 and 7; two residual
-    # restrictions, 9.25 each; two prolongation + post-smoothing sweeps, 12
-    # each; two operator applications, 10 each; the solution update, 8) and
-    # the coarse levels 18.7 (27.25 / 4 per V-cycle, twice, times 4/3)
-    bytes_iter = 104 * 8 * n
+    # vector and coefficient once per pass that needs it: level 0 88 (the two
+    # vector updates fused with pre-smoothing, 8 and 7; two descents, residual
+    # and restriction with the next level's pre-smoothing, 10.25 each; two
+    # ascents, prolongation and post-smoothing, 12.25 each; two operator
+    # applications, 10 each; the solution update, 8) and the coarse levels 15
+    # (22.5 / 4 per V-cycle, twice, times 4/3)
+    bytes_iter = 103 * 8 * n
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -597,11 +598,11 @@ def thermal_leg(Simple, torch, args) -> dict:
     achieved = bytes_iter * its_f / t_f / 1e9
     # the mixed form's bytes per cell and iteration: the V-cycle's levels,
     # factors and iterates in float, the Krylov vectors it reads (p, s) and
-    # the operator of the FP64 matvecs in double: level 0 482 B (update +
-    # pre-smoothing 48 and 40, restrictions 41 each, prolongation + post-
-    # smoothing 52 each, operator applications 76 each, solution update 56),
-    # the coarse levels 74.8 (the FP64 18.7 words in float)
-    bytes_iter_m = 557 * n
+    # the operator of the FP64 matvecs in double: level 0 492 B (update +
+    # pre-smoothing 48 and 40, descents 45 each, ascents 53 each, operator
+    # applications 76 each, solution update 56), the coarse levels 60 (the
+    # FP64 15 words in float)
+    bytes_iter_m = 552 * n
     t_fm = max(r["device_ms"] for r in fwd_m) / 1e3
     t_am = max(r["device_ms"] for r in adj_m) / 1e3
     its_fm = max(r["iterations"] for r in fwd_m)
@@ -633,12 +634,13 @@ def thermal_leg(Simple, torch, args) -> dict:
             "e2e": {"value": float(np.mean(e2e)), "unit": "s", "h2d_bytes_per_step": int(4 * 8 * Nx * Ny),
                     "d2h_bytes_per_step": int(T.nbytes + 16)},
             # launches: assembly, fill, a Galerkin coarsening per coarse level, a
-            # z-factorisation per level, the persistent solver; the adjoint adds
-            # the p-norm, its right-hand side and the sensitivity
+            # z-factorisation per level, the small levels' matrix, the persistent
+            # solver; the adjoint adds the p-norm, its right-hand side and the
+            # sensitivity
             "mixed": mixed,
             "multigrid_levels": levels,
-            "gpu_launches_per_forward": 2 + (levels - 1) + levels + 1,
-            "gpu_launches_per_adjoint": 2 + levels + 1 + 1}
+            "gpu_launches_per_forward": 2 + (levels - 1) + levels + 1 + 1,
+            "gpu_launches_per_adjoint": 2 + levels + 1 + 1 + 1}
 
 
 # ------------------------------------------------------------------ our arm
@@ -724,16 +726,14 @@ def main():
     pcg_iters = kt["pcgIterations"] / max(kt["launches"]["pcg"], 1)
     sa = os.environ.get("CP_PRESSURE_CYCLE") != "pairs"
     if sa:
-        # smoothed aggregation: 38 w per unknown per CG iteration: 18 w for
-        # the CG passes (matvec: read z, p_old, d, fE, fN, write p, Ap; update
-        # fused with level 0's pre-smoothing and residual: read p, Ap, x, r,
-        # 1/d, fE, fN, write x, r', x0, t), 15 w for the rest of level 0
-        # (restriction: read t and three prolongation weights; prolongation:
-        # read x0 and the weights, write t; post-smoothing: read t, r', 1/d,
-        # fE, fN, write y) and 4.5 w for the 9-point coarse levels (about
-        # 36 w per level-1 unknown, a ninth of the unknowns, times 9/8 for
-        # the levels below)
-        words, kname = 38, "k_pcg_sa<float>"
+        # smoothed aggregation: 24 w per unknown per CG iteration: 20 w on level
+        # 0 (matvec: read z, p_old, x, d, fE, fN, write p, Ap, x; update, pre-
+        # smoothing, residual and restriction in one pass: read r, Ap, 1/d, fE,
+        # fN, write r'; prolongation and post-smoothing in one: read r', 1/d,
+        # fE, fN, write z) and 4 w for the 9-point coarse levels (about 32 w
+        # per level-1 unknown, a ninth of the unknowns, times 9/8 for the
+        # levels below)
+        words, kname = 24, "k_pcg_sa<float>"
         cap_bytes, cap_iters = PCG_SA_CAPTURE_BYTES, PCG_SA_CAPTURE_ITERS
     else:
         # 2 x 2 aggregation: 23 w per unknown per CG iteration: 8 w for the CG
@@ -809,7 +809,7 @@ def main():
 
     if rank == 0:
         cb = None if args.no_cpu_baseline else cpu_baseline(case, args.cpu_sample_iters, k64)
-        iters_per_launch = 8
+        iters_per_launch = 7
         t_fp64 = max(t_64)
         # the order puts the metric's own figures (FP64 against mixed, the
         # adjoint) last, where a log that keeps only the end of the line
