@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg(KParams k, Status* st, c
         const TV r = z[c], zz = r / (TV)aP;
         B.r[c] = r;
         z[c] = zz;
+        if (vec) clear_row_ends(B.r, c, j, w);
         acc[1] += (double)r * (double)zz;
     });
     if (!team_reduce(T, target, acc, part, sm)) return;

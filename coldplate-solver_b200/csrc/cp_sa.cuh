@@ -1227,6 +1227,17 @@ __device__ __forceinline__ double sa0_up(const Team& T, const Sa0<TV>& A, const 
     return sa0_up_march(T, A, b, C, y);
 }
 
+// Called for every unknown of the residual when a solve starts: clears the frame
+// columns that share a 16-byte vector with the row's ends.  The passes update and
+// store r in whole vectors, so a solve whose step overflowed leaves NaN there, and
+// nothing else would ever take it out of the sums of the context's later solves.
+template <typename TV>
+__device__ __forceinline__ void clear_row_ends(TV* r, size_t c, int j, int w) {
+    if (j == 1) r[c - 1] = (TV)0;
+    if (j == w)
+        for (int q = 1; q <= (w | (Vec16<TV>::n - 1)) - w; ++q) r[c + q] = (TV)0;
+}
+
 // ---------------------------------------------------------------- the solver
 // The PCG of one pressure-correction solve on a team of CTAs (the whole grid
 // in k_pcg_sa; Few: a group of CTAs in the batched kernel); returns false if a
@@ -1299,6 +1310,7 @@ __device__ __forceinline__ bool pcg_sa(const Team& T, unsigned& target, const KP
         }
         const TV rt = B.rhs[c];
         B.r[c] = rt;
+        clear_row_ends(B.r, c, j, w);
         bb[0] += (double)rt * (double)rt;
     });
     if (!team_reduce(T, target, bb, part, sm)) return false;
