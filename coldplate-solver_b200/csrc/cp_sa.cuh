@@ -84,13 +84,24 @@ struct SaLevel {
     TV* pw[4];
 };
 
+// Entries of a stored row of n unknowns.  Rows laid out with the level's pitch (at
+// least 32) would be up to 32 times as long on a grid a few columns wide, and every
+// CG iteration reads them: 268 MB of 8.4 at 4 x 3070 in double, where an outer
+// iteration took 1003 us with them and takes 274 (4 x 2000: 722 and 225).
+template <typename TV>
+__host__ __device__ __forceinline__ int sa_row(int n) {
+    constexpr int V = 16 / (int)sizeof(TV);
+    return (n + V - 1) / V * V;
+}
+
 template <typename TV>
 struct SaHier {
     int L, Ld;              // levels; levels [0, Ld) run grid-wide, level Ld is solved by bm[Ld]
     SaLevel<TV> lv[kSaMaxLevels];
     TV* dinv0;              // level-0 inverse diagonal
-    // V-cycle matrices of levels [Ld, L): row q (unknown q, row-major) holds
-    // nI x P entries laid out like the level's rows 1 .. nI
+    // V-cycle matrices of levels [Ld, L): row q (unknown q, row-major) holds the
+    // level's nI nJ entries, without its frame, and zeros up to a whole 16 bytes
+    // (sa_row).  Level Ld's right-hand side is stored the same way.
     TV* bm[kSaMaxLevels];
     double omega, w0, wc;   // Jacobi damping, prolongator smoothing weights
     TV* r2;                 // second CG residual buffer (the residual ping-pongs)
@@ -296,11 +307,11 @@ __device__ void sa_invert(const SaLevel<TV>& l, TV* bm, double* work /* 4 x 64 *
             else a[k] = c == s ? -a[k] * ip : a[k] - col[r] * rc;
         }
     }
-    const int len = l.nI * l.P;
+    const int len = sa_row<TV>(n);
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         const int r = r0 + k * (512 / W);
-        if (r < n && c < n) bm[(size_t)r * len + (c / l.nJ) * l.P + 1 + c % l.nJ] = (TV)a[k];
+        if (r < n && c < n) bm[(size_t)r * len + c] = (TV)a[k];
     }
     __syncthreads();
 }
@@ -318,7 +329,7 @@ __device__ __forceinline__ void sa_matrix(const Team& T, const SaLevel<TV>& f, c
     double* t = work;                        // (nI + 2) x (nJ + 2), zero frame
     double* e = t + (f.nI + 2) * Pt;         // coarse correction
     double* rr = e + nc;                     // nine residual entries, then P^T r
-    const int len = f.nI * f.P, lenc = C.nI * C.P, tx = threadIdx.x;
+    const int len = sa_row<TV>(n), lenc = sa_row<TV>(nc), tx = threadIdx.x;
     for (int q = tx; q < (f.nI + 2) * Pt; q += blockDim.x) t[q] = 0.0;
     __syncthreads();
     for (int q = T.rank; q < n; q += T.size) {
@@ -347,13 +358,12 @@ __device__ __forceinline__ void sa_matrix(const Team& T, const SaLevel<TV>& f, c
         }
         __syncthreads();
         for (int c = tx; c < nc; c += blockDim.x) {
-            const size_t at = (size_t)(c / C.nJ) * C.P + 1 + c % C.nJ;
             double s = 0.0;
 #pragma unroll
             for (int k = 0; k < 9; ++k) {
                 const int I = Ia + k / 3 - 1, J = Ja + k % 3 - 1;
                 if (I >= 1 && I <= C.nI && J >= 1 && J <= C.nJ)
-                    s += (double)bc[(size_t)((I - 1) * C.nJ + J - 1) * lenc + at] * rr[16 + k];
+                    s += (double)bc[(size_t)((I - 1) * C.nJ + J - 1) * lenc + c] * rr[16 + k];
             }
             e[c] = s;
         }
@@ -376,7 +386,7 @@ __device__ __forceinline__ void sa_matrix(const Team& T, const SaLevel<TV>& f, c
             double s = 0.0;
 #pragma unroll
             for (int k = 0; k < 9; ++k) s += (double)f.c[k][m] * t[(ii + k / 3 - 1) * Pt + jj + k % 3 - 1];
-            bm[(size_t)q * len + (size_t)(ii - 1) * f.P + jj] =
+            bm[(size_t)q * len + c] =
                 (TV)(t[ii * Pt + jj] + om * ((c == q ? 1.0 : 0.0) - s) / (double)f.c[4][m]);
         }
     }
@@ -388,8 +398,8 @@ template <typename TV>
 __device__ __forceinline__ void sa_apply(const Team& T, const SaLevel<TV>& f, const TV* __restrict__ bm) {
     constexpr int V = Vec16<TV>::n;
     const int lane = threadIdx.x & 31, nw = T.nth() >> 5;
-    const int n = f.nI * f.nJ, len = f.nI * f.P;
-    const TV* b = f.b + f.P;
+    const int n = f.nI * f.nJ, len = sa_row<TV>(n);
+    const TV* b = f.b;
     for (int q = sa_task(T, n, nw); q < n; q += nw) {
         const TV* row = bm + (size_t)q * len;
         double s = 0.0;
@@ -445,7 +455,7 @@ __device__ __forceinline__ void sa_down(const Team& T, const SaLevel<TV>& f, con
         const bool act = col >= 1 && col <= f.nJ;
         const int J = 9 * s + 1 + lane;
         const bool out = lane < 9 && J <= C.nJ;
-        const size_t qc = (size_t)I * C.P + J;
+        const size_t qc = (size_t)I * C.P + J, qb = last ? (size_t)(I - 1) * C.nJ + J - 1 : qc;
         TV x[7];
 #pragma unroll
         for (int r = 0; r < 7; ++r) {
@@ -486,7 +496,7 @@ __device__ __forceinline__ void sa_down(const Team& T, const SaLevel<TV>& f, con
                      h4 = __shfl_sync(0xffffffffu, vH, 3 * lane + 5);
         if (out) {
             const double v = ((h0 + o1) + (o2 + o3)) + h4;
-            C.b[qc] = (TV)v;
+            C.b[qb] = (TV)v;
             if (!last) C.x[qc] = (TV)(om * v / (double)d);
         }
     }
@@ -590,7 +600,7 @@ __device__ __forceinline__ void sa_down_march(const Team& T, const SaLevel<TV>& 
                 if (I >= I0 && out) {
                     const double v = ((h0 + o1) + (o2 + o3)) + h4;
                     const size_t qc = (size_t)I * C.P + J;
-                    C.b[qc] = (TV)v;
+                    C.b[last ? (size_t)(I - 1) * C.nJ + J - 1 : qc] = (TV)v;
                     if (!last) C.x[qc] = (TV)(om * v / (double)d);
                 }
                 ++I;
@@ -906,7 +916,7 @@ __device__ __forceinline__ void sa0_gather(const SaLevel<TV>& C, int s, int I, c
             const size_t qc = (size_t)I * C.P + J;
             const double d = last ? 1.0 : (double)C.c[4][qc];
             const double v = (double)bO[e + 1] + (double)bO[e + 2] + (double)bO[e + 3] + (double)bH[e] + (double)bH[e + 4];
-            C.b[qc] = (TV)v;
+            C.b[last ? (size_t)(I - 1) * C.nJ + J - 1 : qc] = (TV)v;
             if (!last) C.x[qc] = (TV)(omC * v / d);
         }
     }

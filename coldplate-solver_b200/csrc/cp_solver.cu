@@ -550,8 +550,9 @@ cp_status sa_build(cp_ctx* c) {
         for (int q = 0; q < (l < L - 1 ? 16 : 12); ++q)
             if ((s = dalloc_bytes(c, &c->saArr[l][q], ne * c->es)) != CP_OK) return s;
         if (l >= Ld) {
-            const size_t n = (size_t)c->saNI[l] * c->saNJ[l];
-            if ((s = dalloc_bytes(c, &c->saBm[l], n * c->saNI[l] * c->saP[l] * c->es)) != CP_OK) return s;
+            const int n = c->saNI[l] * c->saNJ[l];
+            const size_t row = c->es == 4 ? sa_row<float>(n) : sa_row<double>(n);
+            if ((s = dalloc_bytes(c, &c->saBm[l], n * row * c->es)) != CP_OK) return s;
         }
     }
     if (const char* e = getenv("CP_SA_OMEGA")) c->saOmega = atof(e);
