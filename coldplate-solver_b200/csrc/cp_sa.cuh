@@ -64,6 +64,14 @@ namespace cp {
 constexpr int kSaMaxLevels = 12;
 constexpr int kSaDense = 64;         // coarsest level size, inverted by elimination
 constexpr int kSaApply = 1024;       // levels at or below this size: their V-cycle is a stored matrix
+// The same on a team of CTAs (batches).  A few SMs read the matrix at their own
+// rate and form it a column a CTA, so it is the marches over one more level that
+// are faster.  us an outer iteration, with that level by its matrix and by marches:
+// 24 fields of 90 x 90 (900 unknowns, double), teams of 2 2705 / 961, of 4 1623 /
+// 709, of 8 1702 / 1074, of 16 1648 / 1468, of 32 2471 / 2724; 16 of 247 x 130 (420),
+// of 2 2516 / 2182, of 4 1497 / 1354, of 8 1048 / 1002, of 16 1441 / 1557; 32 of
+// 80 x 40 (378), of 2 781 / 515, of 4 504 / 424, of 8 688 / 711.
+inline int sa_apply_team(int ctas) { return ctas < 4 ? 128 * ctas : ctas < 32 ? 512 : kSaApply; }
 // dynamic shared memory of the solve: the matrix set-up's iterate with its
 // frame (at most 3 x 1026) and coarse correction (at most 342), which the
 // restriction's column buffers (1 KB a warp) share
@@ -106,8 +114,8 @@ struct SaHier {
     double omega, w0, wc;   // Jacobi damping, prolongator smoothing weights
     TV* r2;                 // second CG residual buffer (the residual ping-pongs)
     int reuse;              // rebuild the coarse operators every `reuse` outer iterations (0: only when
-                            // the flag says they are stale)
-    int* dirty;             // device flag: the stored hierarchy is stale (cleared by a rebuild)
+                            // the stored ones are stale)
+    int* built;             // device word: the Ld that the stored hierarchy was built for, 0 when it is stale
     unsigned long long* prof;  // optional per-phase device time (ns, block 0's view), or null
 };
 
@@ -1271,8 +1279,9 @@ __device__ __forceinline__ bool pcg_sa(const Team& T, unsigned& target, const KP
     // prolongation always use the current operator), after a solve that
     // reached the iteration cap with them (early in a run the operator moves
     // fast), and whenever the stored ones are stale (the operator changed
-    // from the host, or another solve such as the adjoint's stored its own)
-    const bool rebuild = *(volatile int*)H.dirty ||
+    // from the host, another solve such as the adjoint's stored its own, or a
+    // batch built its matrices for another level)
+    const bool rebuild = *(volatile int*)H.built != H.Ld ||
                          (H.reuse > 0 && (H.reuse == 1 || (st->iter % H.reuse) == 0 || st->itersP >= k.maxP));
 
     const SaLevel<TV> L0 = H.lv[0];
@@ -1323,6 +1332,9 @@ __device__ __forceinline__ bool pcg_sa(const Team& T, unsigned& target, const KP
         clear_row_ends(B.r, c, j, w);
         bb[0] += (double)rt * (double)rt;
     });
+    // the right-hand side that the matrix is applied to, up to whole 16 bytes
+    if (T.lead())
+        for (int q = H.lv[H.Ld].nI * H.lv[H.Ld].nJ; q < sa_row<TV>(H.lv[H.Ld].nI * H.lv[H.Ld].nJ); ++q) H.lv[H.Ld].b[q] = (TV)0;
     if (!team_reduce(T, target, bb, part, sm)) return false;
     const double rTol = k.pTol * sqrt(bb[0]);
     tick(SA_P_SETUP);
@@ -1420,7 +1432,7 @@ __device__ __forceinline__ bool pcg_sa(const Team& T, unsigned& target, const KP
     });
     if (T.lead()) {
         st->itersP = it;
-        if (rebuild) *H.dirty = 0;
+        if (rebuild) *H.built = H.Ld;
     }
     return true;
 }

@@ -114,18 +114,19 @@ struct cp_ctx {
     // smoothed-aggregation hierarchy (pressureSolverType 4); the 2 x 2 one
     // above stays for type 2 and for batches
     bool useSa = false;
-    int saL = 0, saLd = 0;                   // levels; first level solved by its V-cycle matrix
+    int saL = 0;                             // levels
+    void* saRhs = nullptr;                   // right-hand side of the level that is solved by its matrix
     int saNI[kSaMaxLevels] = {}, saNJ[kSaMaxLevels] = {}, saP[kSaMaxLevels] = {};
     // per level: c[0..8] x y b pw[0..3] (level 0: y, the second CG residual
     // and pw[0..2]; pw only on levels that have a coarser one)
     void* saArr[kSaMaxLevels][16] = {};
     void* saDinv0 = nullptr;                 // level-0 inverse diagonal
-    void* saBm[kSaMaxLevels] = {};           // V-cycle matrices of levels [saLd, saL)
+    void* saBm[kSaMaxLevels] = {};           // V-cycle matrices, from sa_first(c, kSaApply) on
     double saOmega = 0.9, saW0 = 2.0 / 3.0, saWc = 0.8;
     unsigned long long* saProf = nullptr;    // per-phase timers when CP_SA_PROFILE is set
     int saReuse = 4;                         // outer iterations between coarse-operator rebuilds
-    int* saDirty = nullptr;                  // device flag: rebuild the coarse operators on the next solve
-    int* saDirtyAdj = nullptr;               // the same flag for the adjoint's pressure-like solves
+    int* saBuilt = nullptr;                  // device word: what the stored coarse operators were built for (SaHier::built)
+    int* saBuiltAdj = nullptr;               // the same for the adjoint's pressure-like solves
     MgMaps mgMaps;                           // TMA tensor maps of the level-0 tile phases
     // adjoint buffers (allocated on first use, double)
     double* adj[40] = {};
@@ -276,9 +277,7 @@ __global__ void k_alpha(const double* gamma, double* alpha, int M, int N, int P,
 // the smoothed-aggregation coarse operators are rebuilt by the next solve
 // (after a change of geometry or state from the host, or a dispatch call)
 cp_status mark_sa_stale(cp_ctx* c) {
-    if (!c->saDirty) return CP_OK;
-    static const int one = 1;
-    CK(cudaMemcpyAsync(c->saDirty, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    if (c->saBuilt) CK(cudaMemsetAsync(c->saBuilt, 0, sizeof(int), c->stream));
     return CP_OK;
 }
 
@@ -489,12 +488,20 @@ cp_status mg_build(cp_ctx* c) {
     return CP_OK;
 }
 
+// First coarse level of at most `most` unknowns (at least kSaDense)
+int sa_first(const cp_ctx* c, int most) {
+    int l = 1;
+    while ((long long)c->saNI[l] * c->saNJ[l] > most) ++l;
+    return l;
+}
+
+// most: unknowns from which the V-cycle is a stored matrix
 template <typename TV>
-SaHier<TV> sa_hier(cp_ctx* c) {
+SaHier<TV> sa_hier(cp_ctx* c, int most = kSaApply) {
     SaHier<TV> H;
     memset(&H, 0, sizeof(H));
     H.L = c->saL;
-    H.Ld = c->saLd;
+    H.Ld = sa_first(c, most);
     H.omega = c->saOmega;
     H.w0 = c->saW0;
     H.wc = c->saWc;
@@ -502,14 +509,14 @@ SaHier<TV> sa_hier(cp_ctx* c) {
     H.r2 = (TV*)c->saArr[0][11];
     H.dinv0 = (TV*)c->saDinv0;
     H.reuse = c->saReuse;
-    H.dirty = c->saDirty;
+    H.built = c->saBuilt;
     for (int l = 0; l < c->saL; ++l) {
         SaLevel<TV>& v = H.lv[l];
         H.bm[l] = (TV*)c->saBm[l];
         v.nI = c->saNI[l]; v.nJ = c->saNJ[l]; v.P = c->saP[l];
         TV** a = reinterpret_cast<TV**>(c->saArr[l]);
         for (int q = 0; q < 9; ++q) v.c[q] = a[q];
-        v.x = a[9]; v.y = a[10]; v.b = a[11];
+        v.x = a[9]; v.y = a[10]; v.b = l == H.Ld ? (TV*)c->saRhs : a[11];
         for (int q = 0; q < 4; ++q) v.pw[q] = a[12 + q];
     }
     return H;
@@ -517,7 +524,7 @@ SaHier<TV> sa_hier(cp_ctx* c) {
 
 // Level sizes of the smoothed aggregation: 3 x 3 aggregates (rounding up)
 // until at most kSaDense unknowns.  From the first coarse level with at most
-// kSaApply unknowns on, the V-cycle is a stored matrix.
+// kSaApply unknowns (in batches sa_apply_team) on, the V-cycle is a stored matrix.
 cp_status sa_build(cp_ctx* c) {
     int nI = c->d.M - 1, nJ = c->d.N - 2;
     int L = 0;
@@ -529,26 +536,24 @@ cp_status sa_build(cp_ctx* c) {
         nI = sa_coarse(nI); nJ = sa_coarse(nJ);
     }
     c->saL = L;
-    int Ld = 1;
-    while ((long long)c->saNI[Ld] * c->saNJ[Ld] > kSaApply) ++Ld;
-    c->saLd = Ld;
-    c->saP[0] = c->d.P;
+    const int Ld = sa_first(c, kSaApply), Lt = sa_first(c, sa_apply_team(1));
     cp_status s;
+    if ((s = dalloc_bytes(c, &c->saRhs, (size_t)kSaApply * c->es)) != CP_OK) return s;
+    c->saP[0] = c->d.P;
     // level 0: corrected iterate, the second CG residual buffer (its rhs is
     // the CG residual), prolongation weights
     for (int q : {10, 11, 12, 13, 14})
         if ((s = dalloc_bytes(c, &c->saArr[0][q], c->nElem * c->es)) != CP_OK) return s;
     if ((s = dalloc_bytes(c, &c->saDinv0, c->nElem * c->es)) != CP_OK) return s;
-    if ((s = dalloc(c, &c->saDirty, 1)) != CP_OK) return s;
-    if ((s = dalloc(c, &c->saDirtyAdj, 1)) != CP_OK) return s;
-    const int one = 1;
-    CK(cudaMemcpyAsync(c->saDirty, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    if ((s = dalloc(c, &c->saBuilt, 1)) != CP_OK) return s;
+    if ((s = dalloc(c, &c->saBuiltAdj, 1)) != CP_OK) return s;
     for (int l = 1; l < L; ++l) {
         c->saP[l] = ((c->saNJ[l] + 2 + 31) / 32) * 32;
         const size_t ne = (size_t)(c->saNI[l] + 2) * c->saP[l];
-        for (int q = 0; q < (l < L - 1 ? 16 : 12); ++q)
-            if ((s = dalloc_bytes(c, &c->saArr[l][q], ne * c->es)) != CP_OK) return s;
+        // (no pass reads the vectors of the levels below Lt)
+        for (int q = 0; q < 16; ++q)
+            if ((q < 9 || (q >= 12 ? l < L - 1 : q == 10 ? l <= Lt : l < Lt)) &&
+                (s = dalloc_bytes(c, &c->saArr[l][q], ne * c->es)) != CP_OK) return s;
         if (l >= Ld) {
             const int n = c->saNI[l] * c->saNJ[l];
             const size_t row = c->es == 4 ? sa_row<float>(n) : sa_row<double>(n);
@@ -1045,9 +1050,10 @@ cp_status cp_destroy(cp_ctx* c) {
         if (cudaMemcpy(t, c->saProf, sizeof t, cudaMemcpyDeviceToHost) == cudaSuccess) {
             fprintf(stderr, "CP_SA_PROFILE ms: setup %.3f galerkin %.3f matvec %.3f update %.3f dense %.3f", t[SA_P_SETUP] * 1e-6,
                     t[SA_P_GALERKIN] * 1e-6, t[SA_P_MATVEC] * 1e-6, t[SA_P_UPDATE] * 1e-6, t[SA_P_DENSE] * 1e-6);
-            for (int l = 1; l < c->saLd; ++l) fprintf(stderr, " down%d %.3f", l, t[SA_P_DOWN + l] * 1e-6);
-            for (int l = 0; l < c->saLd; ++l) fprintf(stderr, " up%d %.3f", l, t[SA_P_UP + l] * 1e-6);
-            fprintf(stderr, " levels %d grid %d\n", c->saL, c->saLd);
+            const int Ld = sa_first(c, kSaApply);
+            for (int l = 1; l < Ld; ++l) fprintf(stderr, " down%d %.3f", l, t[SA_P_DOWN + l] * 1e-6);
+            for (int l = 0; l < Ld; ++l) fprintf(stderr, " up%d %.3f", l, t[SA_P_UP + l] * 1e-6);
+            fprintf(stderr, " levels %d grid %d\n", c->saL, Ld);
         }
     }
     if (c->graph) cudaGraphExecDestroy(c->graph);
@@ -1340,8 +1346,8 @@ cp_status adjoint_pcg(cp_ctx* c, const KParams& k, const double* dE, const doubl
         SaHier<TV> H = sa_hier<TV>(c);
         // the adjoint's operator is fixed over one adjoint solve: built by its
         // first pressure-like solve, reused by the rest (the caller marks both
-        // flags stale at the start)
-        H.dirty = c->saDirtyAdj;
+        // stale at the start)
+        H.built = c->saBuiltAdj;
         H.reuse = 0;
         CK(launch_coop_cfg(k_pcg_sa<TV>, c->gMg, kMgThreads, kSaSmem, c->stream, k, c->adjSt, dE, dN, B, H, out,
                            c->adjPart, c->adjBar));
@@ -1436,9 +1442,8 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
     if (s != CP_OK) return s;
     // the adjoint's pressure-like solves store their own coarse operators:
     // built once for this solve, and the forward's rebuilt after it
-    if (c->saDirtyAdj) {
-        static const int one = 1;
-        CK(cudaMemcpyAsync(c->saDirtyAdj, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    if (c->saBuiltAdj) {
+        CK(cudaMemsetAsync(c->saBuiltAdj, 0, sizeof(int), c->stream));
         if ((s = mark_sa_stale(c)) != CP_OK) return s;
     }
     CK(cudaEventRecord(c->ev0, c->stream));
@@ -2096,7 +2101,7 @@ BField<TC> batch_field(cp_ctx* c) {
 }
 
 template <typename TC>
-BFieldSa<TC> batch_field_sa(cp_ctx* c) {
+BFieldSa<TC> batch_field_sa(cp_ctx* c, int ctas) {
     BFieldSa<TC> bf;
     memset(&bf, 0, sizeof(bf));
     bf.k = c->k;
@@ -2107,19 +2112,11 @@ BFieldSa<TC> batch_field_sa(cp_ctx* c) {
     bf.V = mom_sys<TC>(c, 1);
     bf.xU0 = (TC*)c->xb[0]; bf.xU1 = (TC*)c->xb[1]; bf.xV0 = (TC*)c->xb[2]; bf.xV1 = (TC*)c->xb[3];
     bf.B = pcg_bufs<TC>(c);
-    bf.H = sa_hier<TC>(c);
+    bf.H = sa_hier<TC>(c, sa_apply_team(ctas));
     bf.H.prof = nullptr;
     bf.partJ = c->partJ; bf.partM = c->partM; bf.partP = c->partP;
     bf.hist = c->hist; bf.histCap = c->histCap; bf.dpWin = c->dpWin;
     return bf;
-}
-
-cp_status batch_set_team(cp_batch* b, int ctas) {
-    if (ctas < 1 || ctas > b->grid) return fail(CP_ERR_BAD_PARAM, "team of %d CTAs (1..%d)", ctas, b->grid);
-    b->team = ctas;
-    b->nTeams = b->grid / ctas;
-    if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
-    return CP_OK;
 }
 
 template <typename TC, bool Mixed>
@@ -2218,7 +2215,7 @@ template <typename TC>
 cp_status batch_upload_fields(cp_batch* b) {
     if (b->teamMode) {
         std::vector<BFieldSa<TC>> h;
-        for (cp_ctx* c : b->f) h.push_back(batch_field_sa<TC>(c));
+        for (cp_ctx* c : b->f) h.push_back(batch_field_sa<TC>(c, b->team));
         CK(cudaMemcpyAsync(b->dF, h.data(), h.size() * sizeof(BFieldSa<TC>), cudaMemcpyHostToDevice, b->stream));
         // queue order: largest field first (cells), so the last fields a team
         // takes are the short ones
@@ -2234,6 +2231,15 @@ cp_status batch_upload_fields(cp_batch* b) {
     }
     CK(cudaStreamSynchronize(b->stream));
     return CP_OK;
+}
+
+// (the level that the fields solve by its matrix goes with the team)
+cp_status batch_set_team(cp_batch* b, int ctas) {
+    if (ctas < 1 || ctas > b->grid) return fail(CP_ERR_BAD_PARAM, "team of %d CTAs (1..%d)", ctas, b->grid);
+    b->team = ctas;
+    b->nTeams = b->grid / ctas;
+    if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
+    return b->mixed ? batch_upload_fields<float>(b) : batch_upload_fields<double>(b);
 }
 
 cp_status batch_sync_fields(cp_batch* b) {
@@ -2389,10 +2395,10 @@ cp_status cp_batch_create(cp_ctx* const* fields, int n, cp_batch** out) {
             return bail(s);
         if ((s = batch_balloc(b, (void**)&b->dRunning, sizeof(int))) != CP_OK) return bail(s);
     }
-    s = b->mixed ? batch_upload_fields<float>(b) : batch_upload_fields<double>(b);
-    if (s != CP_OK) return bail(s);
     if ((s = batch_set_tile(b, b->R, b->C)) != CP_OK) return bail(s);
-    if (b->teamMode && (s = batch_set_team(b, std::min(kBatchTeamDefault, b->grid))) != CP_OK) return bail(s);
+    if (b->teamMode) s = batch_set_team(b, std::min(kBatchTeamDefault, b->grid));
+    else s = b->mixed ? batch_upload_fields<float>(b) : batch_upload_fields<double>(b);
+    if (s != CP_OK) return bail(s);
     *out = b;
     return CP_OK;
 }
