@@ -115,6 +115,8 @@ SIGNATURES = {
     "cp_read_fluid_params": (_I, [ctypes.c_char_p, ctypes.POINTER(CpParams)]),
     "cp_create": (_I, [ctypes.POINTER(CpParams), ctypes.POINTER(_vp)]),
     "cp_destroy": (_I, [_vp]),
+    "cp_release_cached_memory": (_I, []),
+    "cp_set_cached_memory_limit": (_I, [ctypes.c_size_t, ctypes.c_size_t]),
     "cp_set_cell_type": (_I, [_vp, _dp, _L, _L, _L, _L]),
     "cp_set_gamma": (_I, [_vp, _dp, _L, _L, _L, _L]),
     "cp_read_geometry": (_I, [_vp, ctypes.c_char_p]),

@@ -41,6 +41,19 @@ def make_params(**knobs) -> nat.CpParams:
     return p
 
 
+def release_cached_memory() -> None:
+    """Give the memory kept from destroyed contexts back to the device (and the
+    host), for another allocator of the process, PyTorch's say, which cannot ask
+    for it itself."""
+    nat.check(nat.lib().cp_release_cached_memory())
+
+
+def set_cached_memory_limit(device_bytes: int, host_bytes: int) -> None:
+    """Most device and pinned host memory to keep from destroyed contexts, a CUDA
+    context (4 GB and 256 MB at first; 0: none)."""
+    nat.check(nat.lib().cp_set_cached_memory_limit(device_bytes, host_bytes))
+
+
 class Simple:
     """One field on the GPU.  ``knobs`` are cp_params / SIMPLE.h names."""
 

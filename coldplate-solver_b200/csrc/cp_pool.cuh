@@ -1,13 +1,16 @@
 // Device and pinned host memory of the solver objects.
 //
-// An object (a flow context, a thermal context) holds some 40 to 200 arrays.
+// An object (a flow context, a thermal context, a batch) holds 10 to 200 arrays.
 // Allocating and freeing each of them costs more than many solves: a context at
 // 811 x 389 took 41 ms to make and destroy for a solve of 110 ms, and now and
 // then seconds.  So an object's arrays are cut from blocks, and a destroyed
 // object's blocks go to a process-wide cache that the next object takes from.
-//   * The cache is bounded (kPoolDeviceMax, kPoolHostMax a CUDA context): the
-//     oldest blocks beyond that are freed.  It is given back when an allocation fails, before
-//     the allocation is tried again, and by cp_release_cached_memory().
+//   * The cache is bounded (kPoolDeviceMax, kPoolHostMax a CUDA context, or
+//     what cp_set_cached_memory_limit() says, 0 for no cache): the oldest
+//     blocks beyond that are freed.  It is given back when an allocation of
+//     this library fails, before that is tried again, and by
+//     cp_release_cached_memory(): other allocators of the process cannot ask
+//     for it.
 //   * A block is handed on only after its last owner's stream was synchronised
 //     (the destroy functions do), so no stream can still be using it, and every
 //     array is cleared on its new owner's stream like a fresh one.
@@ -23,6 +26,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <new>
 #include <vector>
 
 namespace cp {
@@ -102,52 +106,59 @@ public:
             cudaGetLastError();
             return;
         }
-        std::vector<PoolBlock> drop;
-        {
+        bool kept = false;
+        try {
             std::lock_guard<std::mutex> lock(mutex_);
             free_.push_back(b);
-            size_t held = 0;
-            for (const PoolBlock& f : free_)
-                if (f.ctx == ctx) held += f.bytes;
-            for (size_t q = 0; q < free_.size() && held > most_;) {
-                if (free_[q].ctx != ctx) {
-                    ++q;
-                    continue;
-                }
-                drop.push_back(free_[q]);
-                held -= free_[q].bytes;
-                free_.erase(free_.begin() + (long)q);
-            }
+            kept = true;
+        } catch (const std::bad_alloc&) {   // no host memory for the list: the destroy functions do not throw
         }
-        for (const PoolBlock& d : drop) dealloc(d.p);
+        if (kept) trim(ctx, false);
+        else dealloc(b.p);
     }
 
     void release_all() {
         unsigned long long ctx = 0;
-        const bool known = pool_context(&ctx);
-        std::vector<PoolBlock> drop;
+        if (pool_context(&ctx)) trim(ctx, true);
+    }
+
+    // other contexts' blocks are held to it when the next one is given
+    void set_limit(size_t bytes) {
         {
             std::lock_guard<std::mutex> lock(mutex_);
-            for (size_t q = 0; q < free_.size();) {
-                if (known && free_[q].ctx == ctx) {
-                    drop.push_back(free_[q]);
-                    free_.erase(free_.begin() + (long)q);
-                } else {
-                    ++q;
-                }
-            }
+            most_ = bytes;
         }
-        for (const PoolBlock& d : drop) dealloc(d.p);
+        unsigned long long ctx = 0;
+        if (pool_context(&ctx)) trim(ctx, false);
     }
 
 private:
+    // frees the context's oldest blocks beyond the limit, or all of them
+    void trim(unsigned long long ctx, bool all) {
+        for (;;) {
+            PoolBlock old;
+            {
+                std::lock_guard<std::mutex> lock(mutex_);
+                size_t held = 0, first = free_.size();
+                for (size_t q = free_.size(); q-- > 0;)
+                    if (free_[q].ctx == ctx) {
+                        held += free_[q].bytes;
+                        first = q;
+                    }
+                if (first == free_.size() || (!all && held <= most_)) return;
+                old = free_[first];
+                free_.erase(free_.begin() + (long)first);
+            }
+            dealloc(old.p);
+        }
+    }
     cudaError_t alloc(void** p, size_t bytes) { return host_ ? cudaMallocHost(p, bytes) : cudaMalloc(p, bytes); }
     void dealloc(void* p) {
         if (host_) cudaFreeHost(p);
         else cudaFree(p);
     }
     const bool host_;
-    const size_t most_;
+    size_t most_;
     std::mutex mutex_;
     std::vector<PoolBlock> free_;   // oldest first
 };

@@ -1040,6 +1040,12 @@ cp_status cp_release_cached_memory(void) {
     return CP_OK;
 }
 
+cp_status cp_set_cached_memory_limit(size_t device_bytes, size_t host_bytes) {
+    device_cache().set_limit(device_bytes);
+    host_cache().set_limit(host_bytes);
+    return CP_OK;
+}
+
 cp_status cp_destroy(cp_ctx* c) {
     if (!c) return CP_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
@@ -1995,9 +2001,10 @@ extern "C" cp_status cp_selftest_bounded_wait(int kind, double limit_seconds, in
     if (kind != 0 && kind != 1) return fail(CP_ERR_BAD_PARAM, "kind must be 0 (grid barrier) or 1 (mbarrier)");
     if (!(limit_seconds > 0.0) || limit_seconds > 10.0) return fail(CP_ERR_BAD_PARAM, "limit must be in (0, 10] s");
     if (!device_status) return fail(CP_ERR_BAD_PARAM, "NULL argument");
-    void* buf = nullptr;
-    CK(cudaMalloc(&buf, 256));
-    struct Free { void* p; ~Free() { cudaFree(p); } } guard{buf};
+    PoolBlock block;
+    CK(device_cache().acquire(256, &block));
+    struct Free { const PoolBlock& b; ~Free() { device_cache().give(b); } } guard{block};
+    void* const buf = block.p;
     CK(cudaMemset(buf, 0, 256));
     unsigned* counter = static_cast<unsigned*>(buf);
     int* err = reinterpret_cast<int*>(static_cast<char*>(buf) + 128);
@@ -2040,7 +2047,8 @@ struct cp_batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaGraphExec_t graph = nullptr;
     int graphOuter = 0;
-    std::vector<void*> allocs;
+    Arena mem;                   // every device array
+    PoolBlock flagBlock;         // pinned: hFlags
 };
 
 namespace {
@@ -2140,8 +2148,7 @@ cp_status batch_launch_team(cp_batch* b, int nOuter) {
 }
 
 cp_status batch_balloc(cp_batch* b, void** p, size_t bytes) {
-    CK(cudaMalloc(p, std::max<size_t>(bytes, 1)));
-    b->allocs.push_back(*p);
+    CK(b->mem.take(bytes, p));
     CK(cudaMemsetAsync(*p, 0, std::max<size_t>(bytes, 1), b->stream));
     return CP_OK;
 }
@@ -2349,8 +2356,9 @@ cp_status cp_batch_create(cp_ctx* const* fields, int n, cp_batch** out) {
     cp_status s = CP_OK;
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
-        cudaMallocHost(&b->hFlags, 2 * sizeof(int)) != cudaSuccess)
+        host_cache().acquire(4096, &b->flagBlock) != cudaSuccess)
         return bail(fail(CP_ERR_CUDA, "batch stream / events / pinned flags"));
+    b->hFlags = static_cast<int*>(b->flagBlock.p);
     // team mode when every field runs smoothed aggregation (CP_BATCH_TILES=1
     // keeps the tile kernel, which runs the 2 x 2 cycle for every field)
     b->teamMode = !getenv("CP_BATCH_TILES");
@@ -2407,8 +2415,8 @@ cp_status cp_batch_destroy(cp_batch* b) {
     if (!b) return CP_OK;
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
-    for (void* q : b->allocs) cudaFree(q);
-    if (b->hFlags) cudaFreeHost(b->hFlags);
+    b->mem.give_back();
+    host_cache().give(b->flagBlock);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     if (b->stream) cudaStreamDestroy(b->stream);

@@ -173,11 +173,15 @@ cp_status cp_read_fluid_params(const char* path, cp_params* p);
  * and gamma at 1 (all fluid), like SIMPLE::initializeMemory. */
 cp_status cp_create(const cp_params* p, cp_ctx** out);
 cp_status cp_destroy(cp_ctx* ctx);
-/* The memory of destroyed contexts (and thermal contexts) is kept for the next
- * ones, at most 4 GB of device and 256 MB of pinned host memory a CUDA
- * context.  It is given back when an allocation fails, at exit, and by this
- * call (for the current device). */
+/* The memory of destroyed contexts (flow, thermal, batches) is kept for the
+ * next ones, at most 4 GB of device and 256 MB of pinned host memory a CUDA
+ * context.  It is given back when an allocation of this library fails, at exit,
+ * and by cp_release_cached_memory (for the current device).  Another allocator
+ * of the process cannot ask for it: a program that runs one against the
+ * device's limit gives it back first, or sets a lower limit (0: a destroyed
+ * context's memory is freed at once). */
 cp_status cp_release_cached_memory(void);
+cp_status cp_set_cached_memory_limit(size_t device_bytes, size_t host_bytes);
 
 /* Geometry.  cellType: Ny x Nx, 0 fluid .. 1 solid (geometry_fluid.txt,
  * SIMPLE.cpp:633-690, converted as SIMPLE.cpp:695-777).  gamma: Ny x Nx
