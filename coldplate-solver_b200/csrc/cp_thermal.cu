@@ -938,8 +938,8 @@ struct cp_thermal {
     std::vector<ThLevel> lv;          // the hierarchy (level 0: S, lc, linv, z0)
     ThLevel* dlv = nullptr;           // its device copy
     ThHier H{};
-    // CP_PREC_MIXED: float copies of every level for the V-cycle, and the
-    // preconditioned directions in float
+    // CP_PREC_MIXED: float copies of the levels that the V-cycle passes over,
+    // and the preconditioned directions in float
     bool mixed = false;
     size_t matSmem = 0;               // k_th_matrix's dynamic shared memory (bytes)
     std::vector<ThLevelT<float>> lvf;
@@ -982,19 +982,20 @@ cp_status th_narrow(cp_thermal* t, const double* src, float* dst, long long n) {
 
 // The float levels of the mixed-precision V-cycle, shaped like the FP64
 // hierarchy.  Level 0 needs no b (its right-hand side is a Krylov vector)
-// and no y (its output is ph or sh).
+// and no y (its output is ph or sh); level m, which is solved by its matrix,
+// needs nothing else, and the levels behind it nothing at all.
 cp_status th_build_float_hierarchy(cp_thermal* t) {
-    const int L = (int)t->lv.size();
+    const int L = (int)t->lv.size(), m = t->H.m;
     t->lvf.assign(L, ThLevelT<float>{});
-    for (int l = 0; l < L; ++l) {
+    for (int l = 0; l <= m; ++l) {
         const ThLevel& F = t->lv[l];
         ThLevelT<float>& G = t->lvf[l];
         G.nx = F.nx;
         G.ny = F.ny;
         G.ncol = F.ncol;
         G.n = F.n;
-        std::vector<float**> arr = {&G.S.aP, &G.S.aW, &G.S.aE, &G.S.aS, &G.S.aN, &G.S.aB, &G.S.aT,
-                                    &G.lc,   &G.linv, &G.x};
+        std::vector<float**> arr;
+        if (l < m) arr = {&G.S.aP, &G.S.aW, &G.S.aE, &G.S.aS, &G.S.aN, &G.S.aB, &G.S.aT, &G.lc, &G.linv, &G.x};
         if (l > 0) {
             arr.push_back(&G.b);
             arr.push_back(&G.y);
@@ -1009,13 +1010,13 @@ cp_status th_build_float_hierarchy(cp_thermal* t) {
     t->dlvf = static_cast<ThLevelT<float>*>(q);
     TCK(cudaMemcpyAsync(t->dlvf, t->lvf.data(), sizeof(ThLevelT<float>) * L, cudaMemcpyHostToDevice, t->stream));
     t->Hf.L = t->H.L;
-    t->Hf.m = t->H.m;
+    t->Hf.m = m;
     t->Hf.omega = t->H.omega;
     t->Hf.scale0 = t->H.scale0;
     t->Hf.scale = t->H.scale;
     t->Hf.lv = t->dlvf;
     t->Hf.prof = t->H.prof;
-    const size_t nm = (size_t)t->lv[t->H.m].n;
+    const size_t nm = (size_t)t->lv[m].n;
     cp_status s = th_alloc(t, &t->Hf.bm, nm * nm);
     if (s == CP_OK) s = th_alloc(t, &t->phf, (size_t)t->k.n);
     if (s != CP_OK) return s;
@@ -1123,7 +1124,8 @@ cp_status th_objective(cp_thermal* t, double p, double* Tb_max, double* Tb_pnorm
 
 // Column factorisation and the persistent BiCGStab for op x = rhs, op = A or
 // A^T, from V.x; records ev1 after the solve and reads the status back.
-// Mixed precision: the factors are narrowed to the float levels, and the
+// Mixed precision: the factors are narrowed to the float levels above the
+// matrix, and the
 // solve is restarted from its iterate while the FP64 residual it computes
 // on entry (b - op x, not the recursive one) is above rtol, for at most
 // kThRefineRounds launches in all; the iterations add up.
@@ -1135,7 +1137,7 @@ cp_status th_krylov(cp_thermal* t, const double* rhs, const ThVecs& V, ThStatus*
         const int g = (int)std::min<long long>(t->gElem, (F.ncol + kThThreads - 1) / kThThreads);
         k_th_lu<Tr><<<g, kThThreads, 0, t->stream>>>(k.Nz, F);
         TCK(cudaGetLastError());
-        if (t->mixed) {
+        if (t->mixed && (int)l < t->H.m) {
             cp_status s = th_narrow(t, F.lc, t->lvf[l].lc, F.n);
             if (s == CP_OK) s = th_narrow(t, F.linv, t->lvf[l].linv, F.n);
             if (s != CP_OK) return s;
@@ -1353,9 +1355,9 @@ cp_status cp_thermal_solve(cp_thermal* t, cp_thermal_report* rep) {
         k_th_coarsen<<<g, kThThreads, 0, t->stream>>>(k.Nz, t->lv[l], C);
         TCK(cudaGetLastError());
     }
-    // mixed precision: the V-cycle's float copies of every level's operator
+    // mixed precision: the V-cycle's float copies of the operators that it applies
     if (t->mixed)
-        for (size_t l = 0; l < t->lv.size(); ++l) {
+        for (int l = 0; l < t->H.m; ++l) {
             const ThSys& A = t->lv[l].S;
             const ThSysT<float>& B = t->lvf[l].S;
             const double* src[7] = {A.aP, A.aW, A.aE, A.aS, A.aN, A.aB, A.aT};
