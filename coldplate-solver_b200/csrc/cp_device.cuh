@@ -439,10 +439,6 @@ __device__ __forceinline__ void row_segments(const Team& T, int nI, int nJ, F&& 
         fn(i, g * V, g < Ga, lane);
     }
 }
-template <typename TV, typename F>
-__device__ __forceinline__ void row_segments(int nI, int nJ, F&& fn) {
-    row_segments<TV>(Team{(int)blockIdx.x, (int)gridDim.x, nullptr, nullptr}, nI, nJ, static_cast<F&&>(fn));
-}
 
 template <typename TV>
 __device__ __forceinline__ TV from_west(TV v) { return __shfl_up_sync(0xffffffffu, v, 1); }

@@ -355,10 +355,9 @@ __device__ __forceinline__ double jacobi_run(const Dims& d, const MomSys<TC>& S,
 
 // One component of a sweep: its strips and rows, and the runs they are cut into
 struct JacSplit {
-    int S, R, n, rows;
+    int S, R, n;
     __device__ __forceinline__ JacSplit(int V, int i1, int j1, int nw, int both) {
         S = (j1 / V + 30) / 30;
-        rows = i1;
         R = max(1, (i1 * S * both + nw - 1) / nw);
         n = S * ((i1 + R - 1) / R);
     }

@@ -1269,7 +1269,6 @@ __device__ __forceinline__ bool pcg_sa(const Team& T, unsigned& target, const KP
     __shared__ double sm[kReduceSm];
     const Dims d = k.d;
     const int M = d.M, N = d.N, w = N - 2;
-    const int n = (M - 1) * w;
     const int tid = T.tid(), nth = T.nth();
     const SaSplit all{tid, nth};
     const double rho = k.rho, hx = k.hx, hy = k.hy, om = H.omega;
