@@ -92,7 +92,10 @@ public:
             release_all();
             e = alloc(&p, bytes);
         }
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            cudaGetLastError();   // reported here; the next launch's check must not find it
+            return e;
+        }
         *out = PoolBlock{p, bytes, known ? ctx : 0};
         return cudaSuccess;
     }

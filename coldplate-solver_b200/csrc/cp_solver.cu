@@ -1315,6 +1315,8 @@ cp_status cp_get_history(cp_ctx* c, double* rows, int max_rows, int* n_rows) {
 // ======================================================================== adjoint
 namespace {
 
+// adjSt is set last: a call whose allocations failed half-way is not the one that
+// the next call may skip them for
 cp_status adjoint_alloc(cp_ctx* c) {
     if (c->adjSt) return CP_OK;
     for (auto& a : c->adj) {
@@ -1326,7 +1328,6 @@ cp_status adjoint_alloc(cp_ctx* c) {
         if (s != CP_OK) return s;
     }
     cp_status s;
-    if ((s = dalloc(c, &c->adjSt, 1)) != CP_OK) return s;
     if ((s = dalloc(c, &c->adjPart, (size_t)4 * kMaxBlocks)) != CP_OK) return s;
     if ((s = dalloc(c, &c->adjBar, 1)) != CP_OK) return s;
     if (const char* e = getenv("CP_ADJ_RESTART")) c->adjRestart = std::min(std::max(atoi(e), 1), kKryMaxDots - 1);
@@ -1342,7 +1343,7 @@ cp_status adjoint_alloc(cp_ctx* c) {
     c->adjHost = static_cast<double*>(c->adjBlock.p);
     for (auto& e : c->adjEv)
         if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    return CP_OK;
+    return dalloc(c, &c->adjSt, 1);
 }
 
 template <typename TV>

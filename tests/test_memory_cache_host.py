@@ -21,9 +21,10 @@ static unsigned long long context = 1;
 static std::map<void*, size_t> live;
 static char* next_address = reinterpret_cast<char*>(1 << 20);
 
+static cudaError_t last = cudaSuccess;
 static cudaError_t fake_alloc(void** p, size_t bytes) {
     ++calls;
-    if (used + bytes > capacity) return cudaErrorMemoryAllocation;
+    if (used + bytes > capacity) return last = cudaErrorMemoryAllocation;
     *p = next_address;
     next_address += bytes;
     live[*p] = bytes;
@@ -44,7 +45,7 @@ cudaError_t cudaMalloc(void** p, size_t n) { return fake_alloc(p, n); }
 cudaError_t cudaMallocHost(void** p, size_t n) { return fake_alloc(p, n); }
 cudaError_t cudaFree(void* p) { return fake_free(p); }
 cudaError_t cudaFreeHost(void* p) { return fake_free(p); }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() { const cudaError_t e = last; last = cudaSuccess; return e; }
 cudaError_t cudaGetDriverEntryPoint(const char* name, void** f, unsigned long long, cudaDriverEntryPointQueryResult* q) {
     *f = name[5] == 'G' && name[8] == 'C' ? reinterpret_cast<void*>(current) : reinterpret_cast<void*>(id);
     *q = cudaDriverEntryPointSuccess;
@@ -99,6 +100,7 @@ int main(int argc, char** argv) {
         cp::Arena d;
         CHECK(take(d, 200) == cudaErrorMemoryAllocation);
         CHECK(used == 900 * MB);
+        CHECK(cudaGetLastError() == cudaSuccess);   // nothing left for the next launch's check
     } else if (what == "context") {
         cp::Arena a, b;
         CHECK(take(a, 100) == cudaSuccess);
