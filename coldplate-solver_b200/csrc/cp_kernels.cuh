@@ -2,19 +2,23 @@
 //
 // One outer iteration (SIMPLE::calculateStep, iterations.cpp:82-659, with
 // momentumSolverType 1) runs as:
-//   k_bc        velocity + pressure boundary conditions     boundaries.cpp:50-146
+//   k_bc        velocity + pressure boundary conditions;     boundaries.cpp:50-146
+//               clears the counters of the kernels behind it
 //   k_assemble  U and V momentum coefficients, fused:        momentum_solver.cpp:197-314
 //               FOU upwinding, half-cell walls, Brinkman,    boundaries.cpp:148-206
 //               2.5-D sink, relaxation, SOU correction,      convection.cpp:53-186
 //               dE/dN, boundary neighbours folded into b
-//   k_jacobi    persistent: Jacobi sweeps of U and V         jacobi_solver.cpp:44-67
-//               together, stop rule per component, then
+//   k_jacobi    persistent: Jacobi sweeps of U and V, stop   jacobi_solver.cpp:44-67
+//               rule per component, then
 //               scatter/clamp/max-change and BCs on u*, v*   momentum_solver.cpp:335-351
+//               (small grids: k_jacobi_cluster)
 //   k_mass      RMS of u*-u, v*-v; mass imbalance; PCG rhs   iterations.cpp:499-533,
 //                                                            pressure_solver.cpp:471-488,733-742
-//   k_pcg       persistent: matrix-free Jacobi-PCG on p'     pressure_solver.cpp:121-184
-//   k_correct   p += pAlpha p'; u, v corrections + clamps    iterations.cpp:556-597
-//   k_bc        boundary conditions again                    iterations.cpp:567,599
+//   the pressure solve on p', by type and size: k_pcg or     pressure_solver.cpp:121-184,
+//               k_pcg_cluster (cp_pcg.cuh), k_pcg_sa         747-766
+//               (cp_sa.cuh), k_pcg_mg (cp_mg.cuh)
+//   k_correct   p += pAlpha p'; u, v corrections + clamps,   iterations.cpp:556-599
+//               with the boundary conditions that copy them
 //   k_finalize  pressure-drop sampling, residual reporting,  postprocessing.cpp:103-327,
 //               history row and the stop rules              SIMPLE.cpp:378-491
 //
@@ -577,12 +581,13 @@ __global__ void __launch_bounds__(Seq ? kJacSegThreads : kJacThreads, Seq ? 3 : 
     }
 }
 
-// The same on two clusters, one a component, for grids small enough
-// (cluster_unknowns of both): the six coefficients of a thread's unknowns stay
+// The same on two clusters, one a component, for grids small enough (at most
+// kClMaxK x 512 unknowns of either in a CTA's share of the rows, cluster_unknowns): the six coefficients of a thread's unknowns stay
 // in registers and the iterate, with the neighbour blocks' rows beside a
 // block's, in two buffers of shared memory, so that a sweep is one pass over
 // them and one cluster barrier, which carries the sum too.  Per unknown the
-// arithmetic is jacobi_run's, so u* and v* are the same bits.  us for the
+// arithmetic is jacobi_run's, so the same number of sweeps gives the same bits of
+// u* and v*; the sums that end them are added in another order.  us for the
 // sweeps, here and on every SM: 15.6 and 34.0 at 40 x 17 (11.5 sweeps, double),
 // 27.2 and 56.6 at 256 x 64 (19.5), 38.6 and 75.0 at 253 x 127 (26.6), 40.7 and
 // 60.1 at 400 x 100 (float, 19.4), 47.6 and 61.0 there in double with K = 6.

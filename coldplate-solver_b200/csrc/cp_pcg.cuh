@@ -139,10 +139,11 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg(KParams k, Status* st, c
 // no global memory at all: three cluster barriers of 0.3 us each, two of which
 // carry the sums.  What bounds it is the chain of barriers, warp sums and
 // shared-memory round trips, and 16 SMs' double-precision divisions as K grows.
-// us an iteration, here and on every SM (double): 2.9 and 6.5 at 40 x 17, 3.7
-// and 7.0 at 256 x 64, 4.5 and 7.2 at 256 x 128, 6.3 and 7.3 at 440 x 110 with
-// K = 6.  At K = 8 (512 x 128) registers spill and both take 7.4, so the line is
-// at K = 6, 49152 unknowns.
+// us an iteration, here and on every SM (double): 2.9 and 6.3 at 40 x 17, 3.7
+// and 7.0 at 256 x 64, 4.4 and 7.1 at 256 x 128, 5.4 and 7.2 at 438 x 110 with
+// K = 6 (float: 2.9 and 6.1, 3.5 and 6.4, 4.1 and 6.6, 4.6 and 7.1).  At K = 8
+// (512 x 128) registers spill and both take 7.4, so the line is at K = 6: a
+// sixteenth of the rows, rounded up, times the unknowns of one at most 3072.
 // Bytes of shared memory: p on R + 2 rows, the north faces on R + 1 and the
 // east faces on R, each w + 2 wide.
 inline size_t pcg_cl_smem(int M, int N, size_t es) { return (size_t)(3 * cluster_rows(M - 1) + 3) * N * es; }

@@ -42,15 +42,16 @@
 //     20 words an unknown and CG iteration on level 0 against 33 with each
 //     of them stored;
 //   * the V-cycle from the first level with at most kSaApply unknowns down
-//     is one symmetric matrix, formed whenever the coarse operators are
-//     rebuilt and applied by the whole grid, one warp a row;
+//     (fewer on a team of CTAs, sa_apply_team) is one symmetric matrix, formed
+//     whenever the coarse operators are rebuilt and applied by the whole grid,
+//     one warp a row;
 //   * block sums ride on the barrier that follows them (team_reduce).
 // Barriers a CG iteration: 4 + 2 (grid-wide coarse levels), 10 at
 // 2048 x 1024 and 6 at 253 x 127, against 14 and 10 with a barrier between
-// every two steps and the small levels on one CTA.  Measured a pressure solve
-// (17.1, 17.1, 17.2, 15.6 CG iterations), before and after: 2048 x 1024 float
-// 2.52 and 1.70 ms, double 3.66 and 2.10 ms; 811 x 389 float 1.06 and 0.65 ms;
-// 253 x 127 double 0.70 and 0.37 ms.
+// every two steps and the small levels on one CTA.  Measured a pressure solve,
+// the mean of a density field's first 20 outer iterations (17.1, 17.1, 17.2, 15.6
+// CG iterations), before and after: 2048 x 1024 float 2.52 and 1.56 ms, double 3.66
+// and 2.11 ms; 811 x 389 float 1.06 and 0.64 ms; 253 x 127 double 0.70 and 0.37 ms.
 // The coarse operators are rebuilt every `reuse` outer iterations; the CG
 // matvec and level 0's smoother and prolongation always use the current
 // operator.  The CG recurrences, the |p.Ap| < 1e-20 exit and AMGCL's
@@ -683,7 +684,10 @@ __device__ __forceinline__ void sa_up_march(const Team& T, const SaLevel<TV>& f,
 
 // ---------------------------------------------------------------- level 0
 // Level 0's operator: face coefficients fE (east), fN (north), the diagonal
-// d and its inverse.  Every level-0 array is zero on the frame (only the
+// d and its inverse.  The passes form the weights of P in TV from them; the
+// Galerkin product has them from the double set-up, so in float the two P differ by
+// roundings (the CG counts over 60 outer iterations are those of weights rounded
+// once: 751, 781, 825, 841 and 883 from 120 x 60 to 2048 x 1024).  Every level-0 array is zero on the frame (only the
 // unknowns are ever written) and fE / fN are zero on the frame rows and
 // columns, so the passes read neighbours without range checks.  The outlet
 // face (east of the last column, with no unknown behind it) is in d only: with

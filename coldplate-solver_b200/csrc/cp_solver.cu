@@ -1543,9 +1543,12 @@ static cp_status adjoint_impl(cp_ctx* c, double* grad, long rows, long cols, lon
     std::vector<double> part((size_t)2 * nb);
     // The products scatter into y with atomics, which want its lines in the L2.
     // Where the basis vectors read in between leave them there, the kernel that
-    // reads y clears it for the next product and three launches go (253 x 127:
-    // 255 to 240 us an iteration, with the host's wait gone too); at 2048 x 1024
-    // the lines would come back from HBM one atomic at a time (1.8 to 2.1 ms).
+    // reads y clears it for the next product and three launches go; else the lines
+    // come back from HBM one atomic at a time.  us an iteration, cleared by launches
+    // and by the reader: 250 and 245 at 253 x 127 (0.8 MB in the three fields), 324
+    // and 320 at 400 x 200 (1.9), 389 and 388 at 512 x 256 (3.2), 418 and 421 at
+    // 550 x 300 (4.0), 455 and 461 at 640 x 320 (5.0), 525 and 543 at 768 x 384
+    // (7.1), 1.8 and 2.1 ms at 2048 x 1024.
     const int clearY = 3 * bytes <= (size_t(4) << 20);
 
     // the reverse sweeps of both components for the adjoint vector x: the
@@ -1826,7 +1829,7 @@ extern "C" cp_status cp_adjoint_probe(cp_ctx* c, int op, const double* x, double
 // ======================================================================== no-allocation entry point
 // cp_pressure_noalloc: the Jacobi-PCG pressure-correction solve (k_mass +
 // k_pcg<double>, the kernels behind cp_pressure for pressureSolverType 1 on
-// grids too large for one cluster, on any row pitch)
+// grids that no cluster takes, here on any size and row pitch)
 // for callers that cannot allocate device memory.  All of its working
 // memory lives in one file-scope device array of fixed size, below; the
 // caller provides only the inputs and the output.
