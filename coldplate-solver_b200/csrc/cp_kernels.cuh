@@ -38,7 +38,7 @@
 namespace cp {
 
 constexpr int kJacThreads = 512;      // sweeps of both components: one CTA an SM
-constexpr int kJacSegThreads = 256;   // one component after the other: three CTAs an SM
+constexpr int kJacSegThreads = 256;   // one component after the other: up to three CTAs an SM
 
 // ------------------------------------------------------------------ systems
 template <typename TC>
@@ -390,6 +390,12 @@ __device__ __forceinline__ void jacobi_pass(const KParams& k, const MomSys<TC>& 
     }
 }
 
+// Elements a lane of a march over `rows` rows of strips on nw warps: 1, 2 (floats)
+// or 16 bytes
+inline __host__ __device__ int jacobi_width(int N, int rows, int nw, int es) {
+    return (N + 30) / 30 * rows <= nw ? 1 : es == 4 && (N / 2 + 30) / 30 * rows <= nw ? 2 : 16 / es;
+}
+
 // The sweeps of both components (or of one); cur: the buffer that holds the
 // result (-1: the initial iterate), its: the sweeps.  part: 4 doubles a CTA.
 // Returns false if a barrier gave up.
@@ -410,11 +416,11 @@ __device__ __forceinline__ bool jacobi_sweeps(const KParams& k, const MomSys<TC>
         TC* xUn = curU == 0 ? xU1 : xU0;
         TC* xVn = curV == 0 ? xV1 : xV0;
         double acc[2] = {0.0, 0.0};
-        // rows of strips at V = 1 of the components that still sweep
-        const int rows = (onU ? k.d.M - 1 : 0) + (onV ? k.d.M - 2 : 0);
-        if ((k.d.N + 30) / 30 * rows <= nw)
+        // rows of the components that still sweep
+        const int V = jacobi_width(k.d.N, (onU ? k.d.M - 1 : 0) + (onV ? k.d.M - 2 : 0), nw, (int)sizeof(TC));
+        if (V == 1)
             jacobi_pass<TC, Mixed, 1>(k, U, W, u, v, xUc, xUn, xVc, xVn, onU, onV, T, acc);
-        else if (sizeof(TC) == 4 && (k.d.N / 2 + 30) / 30 * rows <= nw)
+        else if (sizeof(TC) == 4 && V == 2)
             jacobi_pass<TC, Mixed, sizeof(TC) == 4 ? 2 : 1>(k, U, W, u, v, xUc, xUn, xVc, xVn, onU, onV, T, acc);
         else
             jacobi_pass<TC, Mixed, Vec16<TC>::n>(k, U, W, u, v, xUc, xUn, xVc, xVn, onU, onV, T, acc);
@@ -432,8 +438,8 @@ __device__ __forceinline__ bool jacobi_sweeps(const KParams& k, const MomSys<TC>
 }
 
 // The sweeps of one component on row segments (32 lane groups of 16 bytes),
-// one segment a warp and trip.  Used where one component's system stays in the
-// L2 and both together do not (host: jacobi_sequential), and in the batched
+// one segment a warp and trip.  Used where both components' systems do not stay
+// in the L2 or one is swept alone (host: jacobi_sequential), and in the batched
 // kernel, whose fields share the L2: there the sweeps of U and then V beat
 // those of both at once (34 sweeps at 2048 x 1024 in float: 0.42 against
 // 0.58 ms; 24 batched fields: 155 against 172 ms), and more warps with fewer

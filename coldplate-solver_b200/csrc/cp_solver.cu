@@ -90,8 +90,7 @@ struct cp_ctx {
     double* hist = nullptr;
     int histCap = 0;
     double* dpWin = nullptr;
-    bool jacSeq = false;               // sweeps of U, then of V (jacobi_sequential)
-    int gJac = 0, gPcg = 0, gElem = 0, gBc = 0, nbMass = 0;
+    int gJac = 0, gJacSeg = 0, gPcg = 0, gElem = 0, gBc = 0, nbMass = 0;
     int clK = 0, clJacK = 0;           // Jacobi-PCG / sweeps on clusters: unknowns a thread (0: on every SM)
     // multigrid hierarchy (pressureSolverType 2 / 4)
     bool useMg = false;
@@ -210,15 +209,32 @@ cp_status validate(const cp_params* p) {
     return CP_OK;
 }
 
-// Whether the Jacobi kernel sweeps U to its end and then V.  A component's
-// sweeps read eight arrays; where those of one component stay in the 126 MB L2
-// and those of both do not, one at a time is faster (2048 x 1024 in float,
-// 67 MB each: 0.42 against 0.58 ms).  Where both fit (131 against 163 us at
-// 811 x 389) and where not even one does (2048 x 1024 in double, 134 MB each:
-// 0.93 against 1.04 ms) both at once are, for their fewer barriers.
-bool jacobi_sequential(const cp_ctx* c) {
-    const size_t one = 8 * c->nElem * c->es, l2 = 100u << 20;
-    return one <= l2 && 2 * one > l2;
+// Whether the Jacobi kernel runs on row segments, U to its end and then V,
+// instead of marching over both between the same barriers.  A component's sweeps
+// read eight arrays.  Where those of both stay in the 126 MB L2 the march is
+// faster for its fewer barriers, where they do not one at a time is.  us a pair of
+// sweeps, march and segments, double: 12.6 and 15.9 at 1024 x 512 (33 MB a
+// component), 17.7 and 18.8 at 1200 x 600 (45), 23.4 and 20.1 at 1300 x 640 (51),
+// 72.9 and 54.7 at 1700 x 1300 (137), 299 and 182 at 4096 x 2048; float: 16.6 and
+// 18.2 at 1300 x 900 (36), 27.5 and 22.6 at 1300 x 1300 (52), 162 and 105 at
+// 4096 x 2048.  One component alone saves no barrier: its march is the faster one
+// only where it takes one float a lane (us a sweep, float: 4.0 and 4.4 at 420 x 130,
+// 4.6 and 4.6 at 400 x 200, 8.2 and 6.2 at 811 x 389, 13.6 and 9.4 at 1400 x 700;
+// double: 4.1 and 3.6 at 420 x 130, 4.5 and 4.0 at 400 x 200, 14.2 and 12.0 at
+// 1400 x 700).
+bool jacobi_sequential(const cp_ctx* c, bool both) {
+    if (2 * 8 * c->nElem * c->es > (100u << 20)) return true;
+    return !both && !(c->es == 4 && jacobi_width(c->d.N, c->d.M - 1, c->numSMs * (kJacThreads / 32), 4) == 1);
+}
+
+// CTAs an SM of the segment form: as many as take a component in one trip of a
+// segment a warp, at most three (us a sweep with 1, 2 and 3, double: 3.6, 4.2, 5.0
+// at 420 x 130, 4.4, 4.0, 4.8 at 400 x 200, 6.0, 5.5, 5.6 at 600 x 300, 18.8, 12.6,
+// 12.0 at 1400 x 700)
+int jacobi_segment_ctas(const cp_ctx* c) {
+    const int V = 16 / (int)c->es, M = c->d.M, N = c->d.N, warps = c->numSMs * (kJacSegThreads / 32);
+    const int segs = std::max((M - 1) * (((N - 2) / V + 32) / 32), (M - 2) * (((N - 1) / V + 32) / 32));
+    return std::min(3, (segs + warps - 1) / warps);
 }
 
 void fill_kparams(cp_ctx* c) {
@@ -663,11 +679,13 @@ cudaError_t launch_pcg(const cp_ctx* c, const KParams& k, Status* st, const doub
 template <typename TC, bool Mixed>
 cudaError_t launch_jacobi(const cp_ctx* c, const MomSys<TC>& U, const MomSys<TC>& V, int doU, int doV, int applyBC) {
     const JacobiOut out{c->uStar, c->vStar};
-    if (c->clJacK == 0)
-        return launch_coop_cfg(c->jacSeq ? k_jacobi<TC, Mixed, true> : k_jacobi<TC, Mixed, false>, c->gJac,
-                               c->jacSeq ? kJacSegThreads : kJacThreads, 0, c->stream, c->k, c->st, U, V,
+    if (c->clJacK == 0) {
+        const bool seg = jacobi_sequential(c, doU && doV);
+        return launch_coop_cfg(seg ? k_jacobi<TC, Mixed, true> : k_jacobi<TC, Mixed, false>, seg ? c->gJacSeg : c->gJac,
+                               seg ? kJacSegThreads : kJacThreads, 0, c->stream, c->k, c->st, U, V,
                                (const double*)c->u, (const double*)c->v, (TC*)c->xb[0], (TC*)c->xb[1], (TC*)c->xb[2],
                                (TC*)c->xb[3], out, (const double*)c->gamma, c->partJ, c->barJ, doU, doV, applyBC);
+    }
     cudaLaunchAttribute attr;
     const cudaLaunchConfig_t cfg = cluster_config(2, jac_cl_smem(c->d, sizeof(TC)), c->stream, &attr);
     return cudaLaunchKernelEx(&cfg, jac_cluster_fn<TC, Mixed>(c->clJacK), c->k, c->st, U, V, (const double*)c->u,
@@ -982,25 +1000,25 @@ cp_status cp_create(const cp_params* prm, cp_ctx** out) {
         if ((s = dalloc_bytes(c, &x, c->nElem * c->es)) != CP_OK) return bail(s);
     for (auto& x : c->pcg)
         if ((s = dalloc_bytes(c, &x, c->nElem * c->es)) != CP_OK) return bail(s);
-    c->jacSeq = jacobi_sequential(c);
     // cooperative grids: every block must be resident
-    int nbJ = 0, nbP = 0;
+    int nbJ = 0, nbS = 0, nbP = 0;
     if (c->prm.precision == CP_PREC_MIXED) {
-        if (c->jacSeq) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<float, true, true>, kJacSegThreads, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<float, true, false>, kJacThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<float, true, false>, kJacThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbS, k_jacobi<float, true, true>, kJacSegThreads, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbP, k_pcg<float>, kPcgThreads, 0);
     } else {
-        if (c->jacSeq) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<double, false, true>, kJacSegThreads, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<double, false, false>, kJacThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbJ, k_jacobi<double, false, false>, kJacThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbS, k_jacobi<double, false, true>, kJacSegThreads, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbP, k_pcg<double>, kPcgThreads, 0);
     }
-    if (nbJ < 1 || nbP < 1) return bail(fail(CP_ERR_CUDA, "cooperative kernels do not fit on an SM"));
-    c->gJac = c->numSMs * (c->jacSeq ? std::min(nbJ, 3) : 1);
+    if (nbJ < 1 || nbS < 1 || nbP < 1) return bail(fail(CP_ERR_CUDA, "cooperative kernels do not fit on an SM"));
+    c->gJac = c->numSMs;
+    c->gJacSeg = c->numSMs * std::min(nbS, jacobi_segment_ctas(c));
     c->gPcg = c->numSMs;
     c->gElem = c->numSMs * 4;
     c->gBc = std::min(c->numSMs, (std::max(M, N) + kThreads) / kThreads);   // one boundary entry a thread
     c->nbMass = c->numSMs * 4;
-    if (c->gJac > kMaxBlocks || c->gPcg > kMaxBlocks || c->nbMass > kMaxBlocks)
+    if (std::max(c->gJac, c->gJacSeg) > kMaxBlocks || c->gPcg > kMaxBlocks || c->nbMass > kMaxBlocks)
         return bail(fail(CP_ERR_CUDA, "too many SMs for the partial-sum buffers"));
     c->useMg = (prm->pressureSolverType == 2 || prm->pressureSolverType == 4);
     if (c->useMg && (s = mg_build(c)) != CP_OK) return bail(s);
@@ -1011,7 +1029,7 @@ cp_status cp_create(const cp_params* prm, cp_ctx** out) {
     if (c->useSa && (s = sa_build(c)) != CP_OK) return bail(s);
     c->clJacK = c->prm.precision == CP_PREC_MIXED ? jac_cluster_k<float, true>(c->d) : jac_cluster_k<double, false>(c->d);
     if (!c->useMg) c->clK = c->prm.precision == CP_PREC_MIXED ? pcg_cluster_k<float>(c->d) : pcg_cluster_k<double>(c->d);
-    if ((s = dalloc(c, &c->partJ, (size_t)4 * c->gJac)) != CP_OK) return bail(s);
+    if ((s = dalloc(c, &c->partJ, (size_t)4 * std::max(c->gJac, c->gJacSeg))) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->partM, (size_t)4 * c->nbMass)) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->partP, (size_t)4 * std::max(c->gPcg, c->gMg))) != CP_OK) return bail(s);
     if ((s = dalloc(c, &c->barJ, 1)) != CP_OK) return bail(s);
