@@ -87,7 +87,7 @@ constexpr size_t kSaSmem = sizeof(double) * (3 * (kSaApply + 2) + (kSaApply + 2)
 // one; zero on the frame; level 0's only for the Galerkin product).
 template <typename TV>
 struct SaLevel {
-    int nI, nJ, P;
+    int nI, nJ, P, Pb;      // Pb: pitch of b, P but on the level that is solved by its matrix
     TV* c[9];
     TV *x, *y, *b;          // pre-smoothed iterate, corrected iterate, rhs
     TV* pw[4];
@@ -110,7 +110,8 @@ struct SaHier {
     TV* dinv0;              // level-0 inverse diagonal
     // V-cycle matrices of levels [Ld, L): row q (unknown q, row-major) holds the
     // level's nI nJ entries, without its frame, and zeros up to a whole 16 bytes
-    // (sa_row).  Level Ld's right-hand side is stored the same way.
+    // (sa_row).  Level Ld's right-hand side is stored the same way: b there is
+    // nJ + 1 elements ahead of it and Pb = nJ, so that unknown (i, j) is at i Pb + j.
     TV* bm[kSaMaxLevels];
     double omega, w0, wc;   // Jacobi damping, prolongator smoothing weights
     TV* r2;                 // second CG residual buffer (the residual ping-pongs)
@@ -408,17 +409,32 @@ __device__ __forceinline__ void sa_apply(const Team& T, const SaLevel<TV>& f, co
     constexpr int V = Vec16<TV>::n;
     const int lane = threadIdx.x & 31, nw = T.nth() >> 5;
     const int n = f.nI * f.nJ, len = sa_row<TV>(n);
-    const TV* b = f.b;
+    const TV* b = f.b + (f.nJ + 1);
     for (int q = sa_task(T, n, nw); q < n; q += nw) {
         const TV* row = bm + (size_t)q * len;
         double s = 0.0;
-#pragma unroll 4
-        for (int e = lane * V; e < len; e += 32 * V) {
-            const Vec16<TV> m = ld16(row + e), v = ld16(b + e);
-            TV u = m.v[0] * v.v[0];
+        // several loads in flight whatever the row's length: a loop of single ones
+        // waited for each on rows shorter than four trips (0.6 and 1.1 us a CG
+        // iteration at 1200 x 600 and 20000 x 100); in double four of m and b at
+        // once cost the other passes registers (2048 x 1024: 1836 and 1814 us a
+        // solve, float the other way round)
+        constexpr int U = sizeof(TV) == 4 ? 4 : 2;
+#pragma unroll 2
+        for (int e = lane * V; e < len; e += 32 * U * V) {
+            Vec16<TV> m[U], v[U];
 #pragma unroll
-            for (int k = 1; k < V; ++k) u += m.v[k] * v.v[k];
-            s += (double)u;
+            for (int h = 0; h < U; ++h) {
+                const bool on = e + 32 * V * h < len;
+                m[h] = on ? ld16(row + e + 32 * V * h) : zero16<TV>();
+                v[h] = on ? ld16(b + e + 32 * V * h) : zero16<TV>();
+            }
+#pragma unroll
+            for (int h = 0; h < U; ++h) {
+                TV u = m[h].v[0] * v[h].v[0];
+#pragma unroll
+                for (int k = 1; k < V; ++k) u += m[h].v[k] * v[h].v[k];
+                s += (double)u;
+            }
         }
         s = warp_sum(s);
         if (lane == 0) f.y[(size_t)(1 + q / f.nJ) * f.P + 1 + q % f.nJ] = (TV)s;
@@ -464,7 +480,7 @@ __device__ __forceinline__ void sa_down(const Team& T, const SaLevel<TV>& f, con
         const bool act = col >= 1 && col <= f.nJ;
         const int J = 9 * s + 1 + lane;
         const bool out = lane < 9 && J <= C.nJ;
-        const size_t qc = (size_t)I * C.P + J, qb = last ? (size_t)(I - 1) * C.nJ + J - 1 : qc;
+        const size_t qc = (size_t)I * C.Pb + J;
         TV x[7];
 #pragma unroll
         for (int r = 0; r < 7; ++r) {
@@ -505,7 +521,7 @@ __device__ __forceinline__ void sa_down(const Team& T, const SaLevel<TV>& f, con
                      h4 = __shfl_sync(0xffffffffu, vH, 3 * lane + 5);
         if (out) {
             const double v = ((h0 + o1) + (o2 + o3)) + h4;
-            C.b[qb] = (TV)v;
+            C.b[qc] = (TV)v;
             if (!last) C.x[qc] = (TV)(om * v / (double)d);
         }
     }
@@ -608,8 +624,8 @@ __device__ __forceinline__ void sa_down_march(const Team& T, const SaLevel<TV>& 
                              h4 = __shfl_sync(0xffffffffu, vH, 3 * lane + 5);
                 if (I >= I0 && out) {
                     const double v = ((h0 + o1) + (o2 + o3)) + h4;
-                    const size_t qc = (size_t)I * C.P + J;
-                    C.b[last ? (size_t)(I - 1) * C.nJ + J - 1 : qc] = (TV)v;
+                    const size_t qc = (size_t)I * C.Pb + J;
+                    C.b[qc] = (TV)v;
                     if (!last) C.x[qc] = (TV)(om * v / (double)d);
                 }
                 ++I;
@@ -925,10 +941,10 @@ __device__ __forceinline__ void sa0_gather(const SaLevel<TV>& C, int s, int I, c
     for (int h = 0; h < (9 * V + 31) / 32; ++h) {
         const int m = lane + 32 * h, J = 9 * V * s + 1 + m, e = V + 3 * m;
         if (m < 9 * V && J <= C.nJ) {
-            const size_t qc = (size_t)I * C.P + J;
+            const size_t qc = (size_t)I * C.Pb + J;
             const double d = last ? 1.0 : (double)C.c[4][qc];
             const double v = (double)bO[e + 1] + (double)bO[e + 2] + (double)bO[e + 3] + (double)bH[e] + (double)bH[e + 4];
-            C.b[last ? (size_t)(I - 1) * C.nJ + J - 1 : qc] = (TV)v;
+            C.b[qc] = (TV)v;
             if (!last) C.x[qc] = (TV)(omC * v / d);
         }
     }
@@ -1336,8 +1352,10 @@ __device__ __forceinline__ bool pcg_sa(const Team& T, unsigned& target, const KP
         bb[0] += (double)rt * (double)rt;
     });
     // the right-hand side that the matrix is applied to, up to whole 16 bytes
-    if (T.lead())
-        for (int q = H.lv[H.Ld].nI * H.lv[H.Ld].nJ; q < sa_row<TV>(H.lv[H.Ld].nI * H.lv[H.Ld].nJ); ++q) H.lv[H.Ld].b[q] = (TV)0;
+    if (T.lead()) {
+        const SaLevel<TV>& D = H.lv[H.Ld];
+        for (int q = D.nI * D.nJ; q < sa_row<TV>(D.nI * D.nJ); ++q) D.b[D.nJ + 1 + q] = (TV)0;
+    }
     if (!team_reduce(T, target, bb, part, sm)) return false;
     const double rTol = k.pTol * sqrt(bb[0]);
     tick(SA_P_SETUP);

@@ -532,7 +532,12 @@ SaHier<TV> sa_hier(cp_ctx* c, int most = kSaApply) {
         v.nI = c->saNI[l]; v.nJ = c->saNJ[l]; v.P = c->saP[l];
         TV** a = reinterpret_cast<TV**>(c->saArr[l]);
         for (int q = 0; q < 9; ++q) v.c[q] = a[q];
-        v.x = a[9]; v.y = a[10]; v.b = l == H.Ld ? (TV*)c->saRhs : a[11];
+        v.x = a[9]; v.y = a[10]; v.b = a[11];
+        v.Pb = v.P;
+        if (l == H.Ld) {   // the first entry on 16 bytes, nJ + 1 elements behind b
+            v.b = (TV*)c->saRhs + (v.nJ + 32) / 32 * 32 - (v.nJ + 1);
+            v.Pb = v.nJ;
+        }
         for (int q = 0; q < 4; ++q) v.pw[q] = a[12 + q];
     }
     return H;
@@ -554,7 +559,7 @@ cp_status sa_build(cp_ctx* c) {
     c->saL = L;
     const int Ld = sa_first(c, kSaApply), Lt = sa_first(c, sa_apply_team(1));
     cp_status s;
-    if ((s = dalloc_bytes(c, &c->saRhs, (size_t)kSaApply * c->es)) != CP_OK) return s;
+    if ((s = dalloc_bytes(c, &c->saRhs, (size_t)(2 * kSaApply + 64) * c->es)) != CP_OK) return s;
     c->saP[0] = c->d.P;
     // level 0: corrected iterate, the second CG residual buffer (its rhs is
     // the CG residual), prolongation weights
