@@ -225,7 +225,7 @@ __device__ __forceinline__ bool team_sync(const Team& T, unsigned& target) {
 // doubles, written by team_reduce alone.
 constexpr int kReduceSm = 68;
 constexpr int kReduceLoads = 5;   // partials a lane has in flight (148 CTAs: all of them)
-template <int NV>
+template <int NV, int Loads = kReduceLoads>
 __device__ __forceinline__ bool team_reduce(const Team& T, unsigned& target, double (&v)[NV], double* part,
                                             double* sm) {
     static_assert(NV >= 1 && NV <= 2, "two values at most");
@@ -253,14 +253,14 @@ __device__ __forceinline__ bool team_reduce(const Team& T, unsigned& target, dou
         ok = __shfl_sync(0xffffffffu, ok, 0);
 #pragma unroll
         for (int k = 0; k < NV; ++k) t[k] = 0.0;
-        for (int b0 = lane; ok && b0 - lane < T.size; b0 += 32 * kReduceLoads) {
-            double q[kReduceLoads][NV];
+        for (int b0 = lane; ok && b0 - lane < T.size; b0 += 32 * Loads) {
+            double q[Loads][NV];
 #pragma unroll
-            for (int u = 0; u < kReduceLoads; ++u)
+            for (int u = 0; u < Loads; ++u)
 #pragma unroll
                 for (int k = 0; k < NV; ++k) q[u][k] = b0 + 32 * u < T.size ? __ldcg(slot + NV * (b0 + 32 * u) + k) : 0.0;
 #pragma unroll
-            for (int u = 0; u < kReduceLoads; ++u)
+            for (int u = 0; u < Loads; ++u)
 #pragma unroll
                 for (int k = 0; k < NV; ++k) t[k] += q[u][k];
         }

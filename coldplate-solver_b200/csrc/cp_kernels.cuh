@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(256, 4) k_assemble(KParams k, const Status* st
 // while both run, and the sums ride on the barrier (team_reduce).  The sweeps
 // of an outer iteration took 103 us one after the other and take 72 together
 // at 253 x 127 (double, 21 sweeps of one component), 163 and 131 at 811 x 389
-// (float, 30), 1.04 and 0.93 ms at 2048 x 1024 (double, 33).
+// (float, 30).  Larger systems: jacobi_component.
 // A warp takes a run of rows of a strip of 30 V columns: the next row's
 // coefficients are in flight while it works on one, the iterate's rows stay in
 // registers and its horizontal neighbours come by shuffles (lanes 0 and 31
@@ -444,7 +444,7 @@ __device__ __forceinline__ bool jacobi_sweeps(const KParams& k, const MomSys<TC>
 // those of both at once (34 sweeps at 2048 x 1024 in float: 0.42 against
 // 0.58 ms; 24 batched fields: 155 against 172 ms), and more warps with fewer
 // registers beat the prefetch (0.42 against 0.49 ms).
-template <typename TC, bool Mixed, bool IsU>
+template <typename TC, bool Mixed, bool IsU, int Loads = kReduceLoads>
 __device__ __forceinline__ bool jacobi_component(const KParams& k, const MomSys<TC>& S, const double* field,
                                                  TC* x0, TC* x1, double* part, const Team& T, unsigned& target,
                                                  int& cur, int& its) {
@@ -514,7 +514,7 @@ __device__ __forceinline__ bool jacobi_component(const KParams& k, const MomSys<
             }
             if (act) st16(xn + c, o);
         });
-        if (!team_reduce(T, target, acc, part, sm)) return false;
+        if (!team_reduce<1, Loads>(T, target, acc, part, sm)) return false;
         cur = nxt;
         its = s + 1;
         if (acc[0] < lim) break;
@@ -565,8 +565,9 @@ __global__ void __launch_bounds__(Seq ? kJacSegThreads : kJacThreads, Seq ? 3 : 
     const Team T = grid_team(bar, &st->err);
     int curU = -1, curV = -1, itU = 0, itV = 0;
     if constexpr (Seq) {
-        if (doU && !jacobi_component<TC, Mixed, true>(k, U, u, xU0, xU1, part, T, target, curU, itU)) return;
-        if (doV && !jacobi_component<TC, Mixed, false>(k, V, v, xV0, xV1, part, T, target, curV, itV)) return;
+        // (three CTAs an SM have 444 partials, 14 a lane)
+        if (doU && !jacobi_component<TC, Mixed, true, 14>(k, U, u, xU0, xU1, part, T, target, curU, itU)) return;
+        if (doV && !jacobi_component<TC, Mixed, false, 14>(k, V, v, xV0, xV1, part, T, target, curV, itV)) return;
     } else {
         if (!jacobi_sweeps<TC, Mixed>(k, U, V, u, v, xU0, xU1, xV0, xV1, doU, doV, part, T, target, curU, curV, itU, itV))
             return;

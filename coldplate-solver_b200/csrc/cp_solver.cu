@@ -211,19 +211,21 @@ cp_status validate(const cp_params* p) {
 
 // Whether the Jacobi kernel runs on row segments, U to its end and then V,
 // instead of marching over both between the same barriers.  A component's sweeps
-// read eight arrays.  Where those of both stay in the 126 MB L2 the march is
-// faster for its fewer barriers, where they do not one at a time is.  us a pair of
-// sweeps, march and segments, double: 12.6 and 15.9 at 1024 x 512 (33 MB a
-// component), 17.7 and 18.8 at 1200 x 600 (45), 23.4 and 20.1 at 1300 x 640 (51),
-// 72.9 and 54.7 at 1700 x 1300 (137), 299 and 182 at 4096 x 2048; float: 16.6 and
-// 18.2 at 1300 x 900 (36), 27.5 and 22.6 at 1300 x 1300 (52), 162 and 105 at
-// 4096 x 2048.  One component alone saves no barrier: its march is the faster one
-// only where it takes one float a lane (us a sweep, float: 4.0 and 4.4 at 420 x 130,
-// 4.6 and 4.6 at 400 x 200, 8.2 and 6.2 at 811 x 389, 13.6 and 9.4 at 1400 x 700;
-// double: 4.1 and 3.6 at 420 x 130, 4.5 and 4.0 at 400 x 200, 14.2 and 12.0 at
-// 1400 x 700).
+// read eight arrays.  The march is faster for its fewer barriers while those of
+// both stay in the L2, which holds what all SMs read up to about half its 126 MB;
+// beyond, one at a time is.  us a pair of sweeps in solves of type 4 (and of type
+// 1, where one component stops much earlier), march and segments, double: 12.6 and
+// 15.1 (15.2 and 17.0) at 1024 x 512 (33 MB a component), 17.9 and 16.1 (24.8 and
+// 17.8) at 1100 x 560 (38), 28.2 and 21.1 (33.1 and 24.6) at 1400 x 700 (60), 299
+// and 182 at 4096 x 2048; float: 12.4 and 13.8 (21.0 and 17.0) at 1300 x 640 (26),
+// 15.1 and 16.2 (26.5 and 19.3) at 1400 x 700 (30), 16.8 and 16.7 (30.2 and 20.0)
+// at 1400 x 800 (35), 27.0 and 21.6 at 1300 x 1300 (52).  One component alone
+// saves no barrier: its march is the faster one only where it takes one float a
+// lane (us a sweep, float: 4.0 and 4.4 at 420 x 130, 4.6 and 4.5 at 400 x 200, 8.2
+// and 5.7 at 811 x 389, 13.6 and 8.7 at 1400 x 700; double: 4.1 and 3.6 at
+// 420 x 130, 4.5 and 3.6 at 400 x 200, 14.2 and 11.5 at 1400 x 700).
 bool jacobi_sequential(const cp_ctx* c, bool both) {
-    if (2 * 8 * c->nElem * c->es > (100u << 20)) return true;
+    if (2 * 8 * c->nElem * c->es > (68u << 20)) return true;
     return !both && !(c->es == 4 && jacobi_width(c->d.N, c->d.M - 1, c->numSMs * (kJacThreads / 32), 4) == 1);
 }
 
