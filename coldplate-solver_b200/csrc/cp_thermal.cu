@@ -372,9 +372,10 @@ __global__ void k_th_lu(int Nz, ThLevel F) {
 
 // A tile: W = blockDim / Nz whole columns of a level (in column order, so a
 // tile may span rows), a thread a cell: layer kk, tile column c.  The z-solve
-// of a tile runs from shared memory, a thread a column: the cell threads store
-// f = r inv and g = sub inv and lc, so that a step of either sweep is one
-// multiply-add, y = f - g y and x = y - lc x.
+// of a tile runs from shared memory, a thread a column: in double the cell threads
+// store f = r inv and g = sub inv and lc, so that a step of either sweep is one
+// multiply-add, y = f - g y and x = y - lc x.  In float, where sub inv would be a
+// third rounding a step, f = r and g = sub, with inv in x: y = (f - g y) inv.
 template <typename T>
 struct ThTile {
     T *f, *g, *lc, *x;      // [Nz][W] each
@@ -383,13 +384,19 @@ struct ThTile {
     __device__ __forceinline__ int at() const { return kk * W + c; }
     // one cell's share of the z-block M x = r
     __device__ __forceinline__ void put(T r, T inv, T sub, T l) const {
-        f[at()] = r * inv;
-        g[at()] = sub * inv;
+        if constexpr (sizeof(T) == 4) {
+            f[at()] = r;
+            g[at()] = sub;
+            x[at()] = inv;
+        } else {
+            f[at()] = r * inv;
+            g[at()] = sub * inv;
+        }
         lc[at()] = l;
     }
     // after it x holds M^-1 r; the caller may put the next tile's cells at
-    // once, since f, g, lc are not read any more and the next solve's first
-    // barrier orders the reads of x
+    // once: a thread reads and puts its own cell alone, and the next solve's
+    // first barrier comes before the columns' threads read them
     __device__ __forceinline__ void solve(int Nz) const {
         __syncthreads();
         if (threadIdx.x < W) {
@@ -401,6 +408,7 @@ struct ThTile {
 #pragma unroll 4
             for (int k = 0; k < Nz; ++k) {
                 v = F[k * W] - G[k * W] * v;
+                if constexpr (sizeof(T) == 4) v *= X[k * W];
                 X[k * W] = v;
             }
             v = T(0);
@@ -526,17 +534,20 @@ __device__ __forceinline__ void th_up(const ThLevelT<T>& F, const ThLevelT<T>& C
     }
 }
 
-// y = B b on the level that is solved by its matrix, a warp a row
+// y = B b on the level that is solved by its matrix, a warp a row.  Summed in
+// double in either form: the rows of a nearly singular level are long sums of
+// nearly cancelling terms, and sums in float cost mixed adjoints of small plates 5
+// to 10 % more iterations, and two of 500 their convergence.
 template <typename T>
 __device__ __forceinline__ void th_apply(const ThLevelT<T>& F, const T* __restrict__ bm) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = gridDim.x * (blockDim.x >> 5), n = (int)F.n;
     for (int i = wid * gridDim.x + blockIdx.x; i < n; i += nw) {
         const T* row = bm + (size_t)i * n;
-        T s = T(0);
+        double s = 0.0;
 #pragma unroll 16
-        for (int q = lane; q < n; q += 32) s += row[q] * F.b[q];
+        for (int q = lane; q < n; q += 32) s += (double)row[q] * (double)F.b[q];
         s = warp_sum(s);
-        if (lane == 0) F.y[i] = s;
+        if (lane == 0) F.y[i] = T(s);
     }
 }
 
