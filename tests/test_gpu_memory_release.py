@@ -29,11 +29,11 @@ def test_release_and_limit():
     solve()
     assert free() < before       # kept
     release_cached_memory()
-    assert free() == before
+    assert free() >= before
     try:
         set_cached_memory_limit(0, 0)
         solve()
-        assert free() == before
+        assert free() >= before
     finally:
         set_cached_memory_limit(4 << 30, 256 << 20)
     solve()
@@ -49,7 +49,7 @@ def test_a_batch_takes_its_arrays_from_the_cache():
         release = free()
         with Batch(fields) as b:
             b.run(2)
-            assert free() == release
+            assert free() >= release
         assert all(np.isfinite(f.get("p")).all() for f in fields)
     finally:
         for f in fields:
